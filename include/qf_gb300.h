@@ -365,6 +365,13 @@ int qf_probabilities(const void* psi, int n, int layout, double* probs, void* st
 size_t qf_sample_workspace_bytes(int n);
 int qf_sample(const void* psi, int n, int layout, int64_t trials, uint64_t seed, int64_t* counts,
               void* workspace, size_t workspace_bytes, void* stream);
+/* The same draws, listed: draws[j] (int64, device, `trials` entries) = the
+ * basis state of trial j; qf_sample's counts are their histogram.  For few
+ * trials of a large state, where 2^n counts are mostly zeros.  Needs
+ * qf_sample_draws_workspace_bytes(n) of workspace. */
+size_t qf_sample_draws_workspace_bytes(int n);
+int qf_sample_draws(const void* psi, int n, int layout, int64_t trials, uint64_t seed, int64_t* draws,
+                    void* workspace, size_t workspace_bytes, void* stream);
 
 #ifdef __cplusplus
 }

@@ -108,6 +108,8 @@ SIGNATURES = {
     "qf_inner": (_c_int, [_vp, _vp, _c_int, _c_int, _vp, _vp, _sz, _vp]),
     "qf_probabilities": (_c_int, [_vp, _c_int, _c_int, _vp, _vp]),
     "qf_sample": (_c_int, [_vp, _c_int, _c_int, _c_i64, _c_u64, _vp, _vp, _sz, _vp]),
+    "qf_sample_draws_workspace_bytes": (_sz, [_c_int]),
+    "qf_sample_draws": (_c_int, [_vp, _c_int, _c_int, _c_i64, _c_u64, _vp, _vp, _sz, _vp]),
 }
 
 

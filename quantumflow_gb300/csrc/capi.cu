@@ -165,6 +165,11 @@ size_t qf_sample_workspace_bytes(int n) {
   return sample_workspace_bytes(n);
 }
 
+size_t qf_sample_draws_workspace_bytes(int n) {
+  if (n < 1 || n > QF_MAX_QUBITS) return 0;
+  return sample_draws_workspace_bytes(n);
+}
+
 int qf_fill_basis(void* psi, int n, int layout, int64_t index, void* stream) {
   int rc = check_state(psi, n, layout);
   if (rc) return rc;
@@ -453,6 +458,16 @@ int qf_sample(const void* psi, int n, int layout, int64_t trials, uint64_t seed,
   rc = check_ws(workspace, workspace_bytes, sample_workspace_bytes(n));
   if (rc) return rc;
   return sample(psi, n, st(layout), trials, seed, counts, workspace, as_stream(stream));
+}
+
+int qf_sample_draws(const void* psi, int n, int layout, int64_t trials, uint64_t seed, int64_t* draws,
+                    void* workspace, size_t workspace_bytes, void* stream) {
+  int rc = check_state(psi, n, layout);
+  if (rc) return rc;
+  if ((draws == nullptr && trials > 0) || trials < 0) return QF_ERR_INVALID_ARGUMENT;
+  rc = check_ws(workspace, workspace_bytes, sample_draws_workspace_bytes(n));
+  if (rc) return rc;
+  return sample_draws(psi, n, st(layout), trials, seed, draws, workspace, as_stream(stream));
 }
 
 }  // extern "C"

@@ -115,11 +115,9 @@ QF_D void split_any(float v, float& h, float& l) {
 }
 QF_D void split_any(double v, float& h, float& l) { split_d(v, h, l); }
 
-// Block reduction of two float-float accumulators into partials[2*block].
-QF_D void block_reduce2(const FFAcc& a0, const FFAcc& a1, double* partials) {
+// Block reduction of two sums into partials[2*block].
+QF_D void block_reduce2(double v0, double v1, double* partials) {
   __shared__ double sh[2][32];
-  double v0 = (double)a0.s + (double)a0.e;
-  double v1 = (double)a1.s + (double)a1.e;
   v0 = warp_sum(v0);
   v1 = warp_sum(v1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -139,6 +137,25 @@ QF_D void block_reduce2(const FFAcc& a0, const FFAcc& a1, double* partials) {
     partials[2 * blockIdx.x + 1] = s1;
   }
 }
+QF_D void block_reduce2(const FFAcc& a0, const FFAcc& a1, double* partials) {
+  block_reduce2((double)a0.s + (double)a0.e, (double)a1.s + (double)a1.e, partials);
+}
+
+// Complex128 reductions accumulate in FP64.  Splitting a double into a
+// float pair (the float-float accumulators of the other layouts) takes four
+// operations of the FP64 pipe per part, eight an amplitude; the FP64 sums
+// take two (norm), three (diagonal) or four (inner product) and carry 53
+// bits instead of 48.  n = 22, 64 MiB: norm 69 -> 22 us, diagonal
+// 100 -> 31 us.  Four loads in flight per thread.
+template <int KIND>
+QF_D double diag_term(double2 a, const uint16_t* cuts, const double* diag, int64_t x, double acc) {
+  if (KIND == 0) return fma(a.x, a.x, fma(a.y, a.y, acc));
+  const double p = fma(a.x, a.x, a.y * a.y);
+  // an integer below 2^32 in the low word of 2^52: exact without the convert
+  const double c = KIND == 1 ? __hiloint2double(0x43300000, (int)cuts[x]) - 4503599627370496.0 : diag[x];
+  return fma(c, p, acc);
+}
+constexpr int RED_UNROLL = 4;
 
 // kind: 0 = norm2, 1 = expectation with uint16 cuts, 2 = expectation with
 // double diagonal.
@@ -146,6 +163,21 @@ template <int LAY, int KIND>
 __global__ void __launch_bounds__(256) k_reduce_diag(const typename Types<LAY>::E* psi, int64_t namps,
                                                      const uint16_t* cuts, const double* diag,
                                                      double* partials) {
+  if constexpr (LAY == C128) {
+    double s = 0.0;
+    const int64_t nthr = (int64_t)gridDim.x * blockDim.x;
+    int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; x + (RED_UNROLL - 1) * nthr < namps; x += RED_UNROLL * nthr) {
+      double2 a[RED_UNROLL];
+#pragma unroll
+      for (int j = 0; j < RED_UNROLL; ++j) a[j] = psi[x + j * nthr];
+#pragma unroll
+      for (int j = 0; j < RED_UNROLL; ++j) s = diag_term<KIND>(a[j], cuts, diag, x + j * nthr, s);
+    }
+    for (; x < namps; x += nthr) s = diag_term<KIND>(psi[x], cuts, diag, x, s);
+    block_reduce2(s, 0.0, partials);
+    return;
+  }
   FFAcc acc, unused;
   acc.zero();
   unused.zero();
@@ -171,6 +203,17 @@ template <int LAY>
 __global__ void __launch_bounds__(256) k_reduce_inner(const typename Types<LAY>::E* a,
                                                       const typename Types<LAY>::E* b, int64_t namps,
                                                       double* partials) {
+  if constexpr (LAY == C128) {
+    double sr = 0.0, si = 0.0;
+    const int64_t nthr = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < namps; x += nthr) {
+      const double2 u = a[x], v = b[x];
+      sr = fma(u.x, v.x, fma(u.y, v.y, sr));
+      si = fma(u.x, v.y, fma(-u.y, v.x, si));
+    }
+    block_reduce2(sr, si, partials);
+    return;
+  }
   FFAcc re, im;
   re.zero();
   im.zero();
@@ -191,6 +234,17 @@ __global__ void __launch_bounds__(256) k_reduce_inner(const typename Types<LAY>:
 template <int LAY>
 __global__ void __launch_bounds__(256) k_reduce_bit(const typename Types<LAY>::E* psi, int64_t namps, int bit,
                                                     double* partials) {
+  if constexpr (LAY == C128) {
+    double s0 = 0.0, s1 = 0.0;
+    const int64_t nthr = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < namps; x += nthr) {
+      const double2 a = psi[x];
+      double& s = ((x >> bit) & 1) ? s1 : s0;
+      s = fma(a.x, a.x, fma(a.y, a.y, s));
+    }
+    block_reduce2(s0, s1, partials);
+    return;
+  }
   FFAcc p0, p1;
   p0.zero();
   p1.zero();
@@ -303,19 +357,21 @@ int reduce_inner(const void* a, const void* b, int n, int layout, double* out, d
 }
 
 // ------------------------------------------------------ probabilities ------
+template <typename E>
+QF_D double prob_of(E a) {
+  if constexpr (sizeof(a.x) == 8) {
+    return fma(a.x, a.x, a.y * a.y);
+  } else {
+    float h, l;
+    norm2_ff(a, h, l);
+    return (double)h + (double)l;
+  }
+}
 template <int LAY>
 __global__ void k_probs(const typename Types<LAY>::E* psi, int64_t namps, double* probs) {
   const int64_t nthr = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < namps; x += nthr) {
-    if constexpr (LAY == C128) {
-      const double2 a = psi[x];
-      probs[x] = fma(a.x, a.x, a.y * a.y);
-    } else {
-      float h, l;
-      norm2_ff(psi[x], h, l);
-      probs[x] = (double)h + (double)l;
-    }
-  }
+  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < namps; x += nthr)
+    probs[x] = prob_of(psi[x]);
 }
 
 static int grid_for(int64_t items) {
@@ -344,68 +400,115 @@ int probabilities(const void* psi, int n, int layout, double* probs, cudaStream_
 }
 
 // ----------------------------------------------------------- sampling ------
-// Inclusive scan of probabilities in three launches: per-block totals,
-// a single-block scan of the totals, then per-block scans with offsets.
-constexpr int SCAN_BLOCK = 1024;  // amplitudes per scan block (256 threads x 4)
+// Inclusive scan of the probabilities: per-block totals, an exclusive scan
+// of the totals, then a sequential sum within each block from its offset.
+// The order of every sum is fixed (a tree over 256 strided partial sums, a
+// Hillis-Steele scan per 1024 totals with a sequential carry, a sequential
+// sum per 1024 amplitudes), so a seed draws the same outcomes at any launch
+// shape.
+constexpr int SCAN_BLOCK = 1024;  // amplitudes per scan block
+constexpr int SCAN_CHUNK = 1024;  // totals per scan of the totals
 
-__global__ void k_scan_totals(const double* p, int64_t namps, double* totals) {
+// probabilities of one scan block and their total (one pass over the state)
+template <int LAY>
+__global__ void __launch_bounds__(256) k_scan_totals(const typename Types<LAY>::E* psi, double* p, int64_t namps,
+                                                     double* totals) {
   __shared__ double sh[256];
   const int64_t base = (int64_t)blockIdx.x * SCAN_BLOCK;
   double s = 0.0;
-  for (int i = threadIdx.x; i < SCAN_BLOCK; i += blockDim.x) {
+#pragma unroll
+  for (int i = threadIdx.x, k = 0; k < SCAN_BLOCK / 256; ++k, i += 256) {
     const int64_t x = base + i;
-    if (x < namps) s += p[x];
+    if (x < namps) {
+      const double v = prob_of(psi[x]);
+      p[x] = v;
+      s += v;
+    }
   }
   sh[threadIdx.x] = s;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+  for (int w = 128; w >= 32; w >>= 1) {
     if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) totals[blockIdx.x] = sh[0];
-}
-
-// exclusive scan of totals in place (single block, sequential chunks)
-__global__ void k_scan_offsets(double* totals, int64_t nblocks) {
-  __shared__ double sh[1024];
-  double carry = 0.0;
-  for (int64_t c0 = 0; c0 < nblocks; c0 += 1024) {
-    const int64_t i = c0 + threadIdx.x;
-    const double v = i < nblocks ? totals[i] : 0.0;
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {  // Hillis-Steele inclusive scan
-      double t = ((int)threadIdx.x >= o) ? sh[threadIdx.x - o] : 0.0;
-      __syncthreads();
-      sh[threadIdx.x] += t;
-      __syncthreads();
-    }
-    if (i < nblocks) totals[i] = carry + sh[threadIdx.x] - v;
-    const double chunk_total = sh[1023];
-    __syncthreads();
-    carry += chunk_total;
+  if (threadIdx.x < 32) {  // the last five levels pair lanes t and t + w
+    s = sh[threadIdx.x];
+    for (int w = 16; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+    if (threadIdx.x == 0) totals[blockIdx.x] = s;
   }
 }
 
-__global__ void k_scan_blocks(double* p, int64_t namps, const double* offsets) {
-  __shared__ double sh[SCAN_BLOCK];
-  const int64_t base = (int64_t)blockIdx.x * SCAN_BLOCK;
-  for (int i = threadIdx.x; i < SCAN_BLOCK; i += blockDim.x) {
-    const int64_t x = base + i;
-    sh[i] = x < namps ? p[x] : 0.0;
+// inclusive Hillis-Steele scan of each chunk of 1024 totals (one CTA per
+// chunk); sums[c] = the chunk's total
+__global__ void __launch_bounds__(SCAN_CHUNK) k_scan_chunks(const double* totals, double* incl, double* sums,
+                                                            int64_t nblocks) {
+  __shared__ double sh[2][SCAN_CHUNK];
+  const int t = threadIdx.x;
+  const int64_t i = (int64_t)blockIdx.x * SCAN_CHUNK + t;
+  double v = i < nblocks ? totals[i] : 0.0;
+  int cur = 0;
+  sh[0][t] = v;
+  __syncthreads();
+  for (int o = 1; o < SCAN_CHUNK; o <<= 1) {
+    if (t >= o) v += sh[cur][t - o];
+    cur ^= 1;
+    sh[cur][t] = v;
+    __syncthreads();
+  }
+  if (i < nblocks) incl[i] = v;
+  if (t == SCAN_CHUNK - 1) sums[blockIdx.x] = v;
+}
+// exclusive offsets: (carry of the chunks before + inclusive scan) - total
+__global__ void __launch_bounds__(SCAN_CHUNK) k_scan_offsets(double* totals, const double* incl, const double* sums,
+                                                             int64_t nblocks) {
+  __shared__ double carry;
+  if (threadIdx.x == 0) {
+    double c = 0.0;
+    for (unsigned k = 0; k < blockIdx.x; ++k) c += sums[k];
+    carry = c;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {  // sequential within the block: 1024 adds
-    double c = offsets[blockIdx.x];
-    for (int i = 0; i < SCAN_BLOCK; ++i) {
-      c += sh[i];
-      sh[i] = c;
+  const int64_t i = (int64_t)blockIdx.x * SCAN_CHUNK + threadIdx.x;
+  if (i < nblocks) totals[i] = carry + incl[i] - totals[i];
+}
+
+// The sequential sums: one scan block per lane, 32 of them per warp, staged
+// through shared memory in columns of 32 amplitudes (loads and stores stay
+// contiguous; row stride 33 keeps the lanes on distinct banks).  The chain
+// of 1024 dependent FP64 adds is the bound; 32 chains share each issue.
+// n = 22: 311 -> 84 us (one thread of each 256-thread block summed).
+__global__ void __launch_bounds__(32) k_scan_blocks(double* p, int64_t namps, const double* offsets,
+                                                    int64_t nblocks) {
+  __shared__ double sh[32][33];
+  const int lane = threadIdx.x;
+  const int64_t b0 = (int64_t)blockIdx.x * 32;
+  double c = b0 + lane < nblocks ? offsets[b0 + lane] : 0.0;
+  double v[32];
+  auto load = [&](int col) {
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      const int64_t x = (b0 + r) * SCAN_BLOCK + col + lane;
+      v[r] = x < namps ? p[x] : 0.0;
     }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < SCAN_BLOCK; i += blockDim.x) {
-    const int64_t x = base + i;
-    if (x < namps) p[x] = sh[i];
+  };
+  load(0);
+  for (int col = 0; col < SCAN_BLOCK; col += 32) {
+#pragma unroll
+    for (int r = 0; r < 32; ++r) sh[r][lane] = v[r];
+    __syncwarp();
+    if (col + 32 < SCAN_BLOCK) load(col + 32);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      c += sh[lane][j];
+      sh[lane][j] = c;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      const int64_t x = (b0 + r) * SCAN_BLOCK + col + lane;
+      if (x < namps) p[x] = sh[r][lane];
+    }
+    __syncwarp();
   }
 }
 
@@ -417,7 +520,9 @@ QF_D uint64_t mix64(uint64_t z) {
   return z ^ (z >> 31);
 }
 
-__global__ void k_draw(const double* cdf, int64_t namps, int64_t trials, uint64_t seed, int64_t* counts) {
+// one outcome per trial: counted, or written to draws[j]
+template <bool COUNT>
+__global__ void k_draw(const double* cdf, int64_t namps, int64_t trials, uint64_t seed, int64_t* out) {
   const double total = cdf[namps - 1];
   const int64_t nthr = (int64_t)gridDim.x * blockDim.x;
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < trials; j += nthr) {
@@ -429,36 +534,76 @@ __global__ void k_draw(const double* cdf, int64_t namps, int64_t trials, uint64_
       if (cdf[mid] > u) hi = mid;
       else lo = mid + 1;
     }
-    atomicAdd(reinterpret_cast<unsigned long long*>(counts + lo), 1ull);
+    if (COUNT) atomicAdd(reinterpret_cast<unsigned long long*>(out + lo), 1ull);
+    else out[j] = lo;
   }
 }
 
+static int64_t scan_blocks(int n) { return ((int64_t(1) << n) + SCAN_BLOCK - 1) / SCAN_BLOCK; }
+static int64_t scan_chunks(int n) { return (scan_blocks(n) + SCAN_CHUNK - 1) / SCAN_CHUNK; }
+
 size_t sample_workspace_bytes(int n) {
+  return (size_t(1) << n) * 8 + (size_t)scan_blocks(n) * 8 + 256;
+}
+// ... and room for the scan of the totals
+size_t sample_draws_workspace_bytes(int n) {
+  return sample_workspace_bytes(n) + (size_t)(scan_blocks(n) + scan_chunks(n)) * 8;
+}
+
+// the cumulative distribution of |psi|^2 in ws; scratch holds
+// scan_blocks + scan_chunks doubles
+static int sample_cdf(const void* psi, int n, int layout, void* ws, double* scratch, cudaStream_t stream) {
   const int64_t namps = int64_t(1) << n;
-  const int64_t nb = (namps + SCAN_BLOCK - 1) / SCAN_BLOCK;
-  return (size_t)namps * 8 + (size_t)nb * 8 + 256;
+  const int64_t nb = scan_blocks(n), nc = scan_chunks(n);
+  double* cdf = reinterpret_cast<double*>(ws);
+  double* totals = cdf + namps;
+  switch (layout) {
+    case C64:
+      k_scan_totals<C64><<<(unsigned)nb, 256, 0, stream>>>(reinterpret_cast<const float2*>(psi), cdf, namps, totals);
+      break;
+    case C128:
+      k_scan_totals<C128><<<(unsigned)nb, 256, 0, stream>>>(reinterpret_cast<const double2*>(psi), cdf, namps, totals);
+      break;
+    case FF:
+      k_scan_totals<FF><<<(unsigned)nb, 256, 0, stream>>>(reinterpret_cast<const float4*>(psi), cdf, namps, totals);
+      break;
+    default:
+      return QF_ERR_LAYOUT;
+  }
+  k_scan_chunks<<<(unsigned)nc, SCAN_CHUNK, 0, stream>>>(totals, scratch, scratch + nb, nb);
+  k_scan_offsets<<<(unsigned)nc, SCAN_CHUNK, 0, stream>>>(totals, scratch, scratch + nb, nb);
+  k_scan_blocks<<<(unsigned)((nb + 31) / 32), 32, 0, stream>>>(cdf, namps, totals, nb);
+  return check_cuda(cudaGetLastError());
+}
+
+template <bool COUNT>
+static int launch_draw(const void* ws, int n, int64_t trials, uint64_t seed, int64_t* out, cudaStream_t stream) {
+  if (trials <= 0) return QF_OK;
+  int64_t g = (trials + 255) / 256;
+  const int64_t cap = (int64_t)device_sm_count() * 16;
+  if (g > cap) g = cap;
+  k_draw<COUNT><<<(unsigned)g, 256, 0, stream>>>(reinterpret_cast<const double*>(ws), int64_t(1) << n, trials, seed,
+                                                 out);
+  return check_cuda(cudaGetLastError());
 }
 
 int sample(const void* psi, int n, int layout, int64_t trials, uint64_t seed, int64_t* counts,
            void* ws, cudaStream_t stream) {
-  const int64_t namps = int64_t(1) << n;
-  const int64_t nb = (namps + SCAN_BLOCK - 1) / SCAN_BLOCK;
-  double* cdf = reinterpret_cast<double*>(ws);
-  double* totals = cdf + namps;
-  int rc = probabilities(psi, n, layout, cdf, stream);
+  // the scan of the totals borrows the count array (2^n entries, at least
+  // scan_blocks + scan_chunks for every n >= 1) before it is zeroed
+  int rc = sample_cdf(psi, n, layout, ws, reinterpret_cast<double*>(counts), stream);
   if (rc) return rc;
-  k_scan_totals<<<(unsigned)nb, 256, 0, stream>>>(cdf, namps, totals);
-  k_scan_offsets<<<1, 1024, 0, stream>>>(totals, nb);
-  k_scan_blocks<<<(unsigned)nb, 256, 0, stream>>>(cdf, namps, totals);
-  rc = check_cuda(cudaMemsetAsync(counts, 0, (size_t)namps * sizeof(int64_t), stream));
+  rc = check_cuda(cudaMemsetAsync(counts, 0, (size_t(1) << n) * sizeof(int64_t), stream));
   if (rc) return rc;
-  if (trials > 0) {
-    int64_t g = (trials + 255) / 256;
-    const int64_t cap = (int64_t)device_sm_count() * 16;
-    if (g > cap) g = cap;
-    k_draw<<<(unsigned)g, 256, 0, stream>>>(cdf, namps, trials, seed, counts);
-  }
-  return check_cuda(cudaGetLastError());
+  return launch_draw<true>(ws, n, trials, seed, counts, stream);
+}
+
+int sample_draws(const void* psi, int n, int layout, int64_t trials, uint64_t seed, int64_t* draws, void* ws,
+                 cudaStream_t stream) {
+  int rc = sample_cdf(psi, n, layout, ws,
+                      reinterpret_cast<double*>(static_cast<char*>(ws) + sample_workspace_bytes(n)), stream);
+  if (rc) return rc;
+  return launch_draw<false>(ws, n, trials, seed, draws, stream);
 }
 
 // ------------------------------------------------------------ cuts ---------

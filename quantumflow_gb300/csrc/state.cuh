@@ -24,6 +24,9 @@ int probabilities(const void* psi, int n, int layout, double* probs, cudaStream_
 size_t sample_workspace_bytes(int n);
 int sample(const void* psi, int n, int layout, int64_t trials, uint64_t seed, int64_t* counts, void* ws,
            cudaStream_t stream);
+size_t sample_draws_workspace_bytes(int n);
+int sample_draws(const void* psi, int n, int layout, int64_t trials, uint64_t seed, int64_t* draws, void* ws,
+                 cudaStream_t stream);
 int cut_values(uint16_t* cuts, int n, int nedges, const int* edges, cudaStream_t stream);
 int cut_values_weighted(double* cuts, int n, int nedges, const int* edges, const double* w,
                         cudaStream_t stream);
