@@ -96,7 +96,7 @@ size_t qf_reduce_workspace_bytes(int n);
 #define QF_KERNEL_FX_DENSE1 8      /* fixed-point 2x2 sweep (QF_LAYOUT_FX)        */
 #define QF_KERNEL_FX_DENSE2 9      /* fixed-point 4x4 sweep                       */
 #define QF_KERNEL_FX_GROUP 10      /* fixed-point fused pass on a register group  */
-#define QF_KERNEL_FX_ELEMENTWISE 11 /* fixed-point pass of element-wise ops only  */
+#define QF_KERNEL_FX_ELEMENTWISE 11 /* complex128 pass of element-wise ops, or of SWAPs */
 #define QF_KERNEL_FX_SHAPE 12      /* fixed-point straight-line pass (1-2 gates)  */
 #define QF_KERNEL_FX_TENSOR 13     /* complex128 pass on the tensor cores         */
 #define QF_KERNEL_CLASSES 14
@@ -130,7 +130,8 @@ int qf_set_gate_merging(int on);
 /* The pass plan qf_run_circuit would execute, without touching the GPU
  * (diagnostics; no reference counterpart).  For each planned pass, 8 ints
  * in stats[8*b ..]: ops, dense 1-qubit, dense 2-qubit, of those with a lane
- * bit (< 5), element-wise, other, high bits (>= 5), kernel (0 element-wise,
+ * bit (< 5), element-wise, other, high bits (>= 5), kernel (0 element-wise
+ * or qubit-exchange pass,
  * 1 direct single-gate sweep, 2 fused warp-tile or shared-memory pass,
  * 3 group pass, 4 shape pass, 5 one gate in native FP64 inside a
  * QF_LAYOUT_FX circuit, 6 tensor-core complex128 pass).  *nblocks gets the pass count; at most max_blocks

@@ -14,6 +14,8 @@
 //               canonical register place with register-bit exchanges
 //               between them, sign (CZ-like), diagonal and phase ops; G = 0
 //               is a pass of element-wise ops only
+// and, beside the tensor-core passes (tcfx.cu): k_fxphase and k_fxswap
+// (fxphase.cu), runs of diagonal gates and of SWAPs.
 // Each kernel converts the amplitudes it holds to fixed point once, applies
 // its gates, and rounds to FP64 once.
 #include <algorithm>
@@ -21,6 +23,7 @@
 
 #include "engine.cuh"
 #include "fx.cuh"
+#include "fxphase.cuh"
 
 namespace qf {
 
@@ -635,8 +638,11 @@ struct FxBlock {
   bool native = false;  // one op run by the native FP64 kernels
   bool wide = false;    // one unitary gate on 3 or 4 qubits for the tensor-core pass
   int ncoef = 0;
-  int shape = -1;       // table shape of a straight-line pass (-1: other kernels)
+  int shape = -1;       // table shape of a straight-line pass (-1: other kernels), or FXB_*
 };
+constexpr int FXB_TENSOR = -2;  // tensor-core pass
+constexpr int FXB_PHASE = -3;   // phase pass; the window bits are order[0..G)
+constexpr int FXB_SWAP = -4;    // qubit-exchange pass
 
 // A unitary gate on 3 or 4 qubits (dense, or a generalised permutation
 // with unit-modulus entries on 3): the CUDA-core fixed-point kernels do not
@@ -657,9 +663,19 @@ constexpr int FX_G_MAX = 4;
 // while the pass's dense bits stay within gmax; ops the fixed-point kernels
 // do not take close the pass and run alone in native FP64.
 std::vector<FxBlock> fx_split_shapes(std::vector<FxBlock>& blocks, const std::vector<HostOp>& ops);
+void fx_merge(std::vector<HostOp>& ops, int n, int& fusion_k);
+std::vector<FxBlock> fx_blocks(const std::vector<HostOp>& ops, const std::vector<int>& list, int fusion_k,
+                               bool tensor);
 
-std::vector<FxBlock> fx_plan(std::vector<HostOp>& ops, int n, int& fusion_k, bool split = true,
-                             bool wide_ok = false) {
+std::vector<FxBlock> fx_plan(std::vector<HostOp>& ops, int n, int& fusion_k) {
+  fx_merge(ops, n, fusion_k);
+  std::vector<int> all(ops.size());
+  for (size_t i = 0; i < ops.size(); ++i) all[i] = (int)i;
+  std::vector<FxBlock> blocks = fx_blocks(ops, all, fusion_k, false);
+  return fx_split_shapes(blocks, ops);
+}
+
+void fx_merge(std::vector<HostOp>& ops, int n, int& fusion_k) {
   if (fusion_k <= 0) fusion_k = FX_G_MAX;
   if (fusion_k > 1 && g_merge_gates) merge_ops(ops, n);
   // generalised permutations on <= 2 qubits with unit-modulus entries run as
@@ -669,6 +685,25 @@ std::vector<FxBlock> fx_plan(std::vector<HostOp>& ops, int n, int& fusion_k, boo
       op.m = dense_matrix(op);
       op.type = op.k == 1 ? OP_DENSE1 : OP_DENSE2;
     }
+}
+
+// exactly SWAP (a 4x4 permutation by now)
+bool is_swap(const HostOp& op) {
+  if (op.type != OP_DENSE2) return false;
+  static const int to[4] = {0, 2, 1, 3};
+  for (int r = 0; r < 4; ++r)
+    for (int c = 0; c < 4; ++c)
+      if (op.m[r * 4 + c] != cplx(c == to[r] ? 1.0 : 0.0, 0.0)) return false;
+  return true;
+}
+
+// The greedy blocks of the ops `list`.  With `tensor` (planning for the
+// tensor-core passes) the group kernel's limits on element-wise ops do not
+// apply, 3- and 4-qubit unitary gates become blocks of their own, and so do
+// runs of at least three disjoint SWAPs: one exchange pass (n = 23: 70 us)
+// against one tensor-core pass (69 us) per two of them.
+std::vector<FxBlock> fx_blocks(const std::vector<HostOp>& ops, const std::vector<int>& list, int fusion_k,
+                               bool tensor) {
   const int gmax = std::min(fusion_k, FX_G_MAX);
   const bool fuse = fusion_k > 1;
   std::vector<FxBlock> blocks;
@@ -677,14 +712,34 @@ std::vector<FxBlock> fx_plan(std::vector<HostOp>& ops, int n, int& fusion_k, boo
     if (!cur.idx.empty()) blocks.push_back(cur);
     cur = FxBlock();
   };
-  for (int i = 0; i < (int)ops.size(); ++i) {
+  for (size_t li = 0; li < list.size(); ++li) {
+    const int i = list[li];
     const HostOp& op = ops[i];
+    if (tensor && fuse && is_swap(op)) {
+      size_t end = li;
+      uint64_t bits = 0;
+      while (end < list.size() && is_swap(ops[list[end]])) {
+        const HostOp& o = ops[list[end]];
+        const uint64_t m = (uint64_t(1) << o.gb[0]) | (uint64_t(1) << o.gb[1]);
+        if (bits & m) break;
+        bits |= m;
+        ++end;
+      }
+      if (end - li >= 3) {
+        close();
+        cur.idx.assign(list.begin() + li, list.begin() + end);
+        cur.shape = FXB_SWAP;
+        close();
+        li = end - 1;
+        continue;
+      }
+    }
     const FxKind kind = fx_kind(op);
     const int need = fx_coef_count(op);
     if (kind == FXK_NATIVE) {
       close();
       cur.idx.push_back(i);
-      if (wide_ok && tx_wide(op)) {
+      if (tensor && tx_wide(op)) {
         cur.wide = true;
         cur.G = op.k;
         for (int j = 0; j < op.k; ++j) cur.order[j] = op.gb[j];
@@ -698,8 +753,8 @@ std::vector<FxBlock> fx_plan(std::vector<HostOp>& ops, int n, int& fusion_k, boo
     if (kind == FXK_DENSE)
       for (int j = 0; j < op.k; ++j)
         if (std::find(cur.order, cur.order + cur.G, op.gb[j]) == cur.order + cur.G) add[nadd++] = op.gb[j];
-    const bool fits = cur.G + nadd <= gmax && (int)cur.idx.size() < FXG_MAX_OPS / 3 &&
-                      cur.ncoef + need <= FXG_MAX_COEF;
+    const bool fits = cur.G + nadd <= gmax && (tensor || ((int)cur.idx.size() < FXG_MAX_OPS / 3 &&
+                                                          cur.ncoef + need <= FXG_MAX_COEF));
     if (!cur.idx.empty() && (!fuse || !fits)) close();
     if (kind == FXK_DENSE) {
       for (int j = 0; j < op.k; ++j)
@@ -709,7 +764,7 @@ std::vector<FxBlock> fx_plan(std::vector<HostOp>& ops, int n, int& fusion_k, boo
     cur.ncoef += need;
   }
   close();
-  return split ? fx_split_shapes(blocks, ops) : blocks;
+  return blocks;
 }
 
 // Passes made of dense gates and signs only are cut where their next dense
@@ -939,10 +994,11 @@ int fx_group_launch(const FxGroupParams& P, int G, cudaStream_t stream) {
   return check_cuda(cudaGetLastError());
 }
 
-// kernel used by a block: 0 element-wise group pass, 1 direct sweep,
+// kernel used by a block: 0 element-wise or qubit-exchange pass, 1 direct sweep,
 // 3 group pass, 4 shape pass, 5 native FP64 op, 6 tensor-core pass
 int fx_block_kernel(const std::vector<HostOp>& ops, const FxBlock& B) {
-  if (B.shape == -2) return 6;
+  if (B.shape == FXB_TENSOR) return 6;
+  if (B.shape == FXB_PHASE || B.shape == FXB_SWAP) return 0;
   if (B.native) return 5;
   if (B.G == 0) return 0;
   if (B.idx.size() == 1) return 1;
@@ -1271,31 +1327,356 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
 
 }  // namespace
 
-// The passes to run: blocks the tensor-core pass takes stay whole (shape
-// -2), the others are cut into straight-line shapes as before.
+namespace {
+
+// Element-wise ops a phase pass takes: diagonals on one or two qubits,
+// scalars, signs.
+bool phase_op(const HostOp& op) {
+  return op.type == OP_SIGN || op.type == OP_PHASE || (op.type == OP_DIAG && op.k <= 2);
+}
+uint64_t op_bits(const HostOp& op) {
+  uint64_t m = 0;
+  for (int j = 0; j < op.k; ++j) m |= uint64_t(1) << op.gb[j];
+  return m;
+}
+
+// Phase passes for the ops of `list` that touch the bits `must`, each with a
+// window of at most four bits that has a bit of every two-qubit diagonal it
+// takes (the most frequent bits first).  Ops of the list that a pass can
+// take along go with it; the rest stay in `list`.
+void emit_phases(const std::vector<HostOp>& ops, std::vector<int>& list, uint64_t must, std::vector<FxBlock>& out) {
+  auto two = [&](int i) { return ops[i].type == OP_DIAG && ops[i].k == 2; };
+  for (;;) {
+    bool any = false;
+    for (int i : list) any = any || ops[i].type == OP_PHASE || (op_bits(ops[i]) & must);
+    if (!any) return;
+    FxBlock B;
+    B.shape = FXB_PHASE;
+    uint64_t win = 0;
+    for (int pass = 0; pass < 2; ++pass) {  // the ops that must run choose the window first
+      while (B.G < 4) {
+        int count[64] = {0}, best = -1;
+        for (int i : list)
+          if (two(i) && !(op_bits(ops[i]) & win) && (pass == 1 || (op_bits(ops[i]) & must)))
+            for (int j = 0; j < 2; ++j) {
+              const int b = ops[i].gb[j];
+              ++count[b];
+              if (best < 0 || count[b] > count[best] || (count[b] == count[best] && b > best)) best = b;
+            }
+        if (best < 0) break;
+        B.order[B.G++] = best;
+        win |= uint64_t(1) << best;
+      }
+      bool left = false;
+      for (int i : list) left = left || (two(i) && !(op_bits(ops[i]) & win) && (op_bits(ops[i]) & must));
+      if (left) break;
+      if (pass == 0) continue;
+    }
+    std::vector<int> rest;
+    int nsign = 0;
+    for (int i : list) {
+      const bool sign = ops[i].type == OP_SIGN;
+      if ((two(i) && !(op_bits(ops[i]) & win)) || (sign && nsign == FXP_MAX_SIGNS)) {
+        rest.push_back(i);
+        continue;
+      }
+      nsign += sign;
+      B.idx.push_back(i);
+    }
+    list.swap(rest);
+    out.push_back(std::move(B));
+  }
+}
+
+int fx_phase_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, FxPhaseParams& P) {
+  const int G = B.G;
+  std::memset(&P, 0, sizeof(P));
+  P.n = n;
+  P.G = G;
+  int sb[4] = {0, 0, 0, 0};
+  for (int j = 0; j < G; ++j) sb[j] = B.order[j];
+  std::sort(sb, sb + G);
+  uint64_t win = 0;
+  for (int j = 0; j < G; ++j) {
+    P.sbits[j] = (uint8_t)sb[j];
+    win |= uint64_t(1) << sb[j];
+  }
+  auto wpos = [&](int bit) {
+    for (int j = 0; j < G; ++j)
+      if (sb[j] == bit) return j;
+    return -1;
+  };
+  auto tpos = [&](int bit) { return bit - __builtin_popcountll(win & ((uint64_t(1) << bit) - 1)); };
+  for (int c = 0; c < (1 << G); ++c)
+    for (int j = 0; j < G; ++j)
+      if ((c >> j) & 1) P.off[c] |= int64_t(1) << sb[j];
+  Cdd one[5], ratio[5][QF_MAX_QUBITS], kc[16];
+  for (auto& v : one) v.re.hi = 1.0;
+  for (auto& row : ratio)
+    for (auto& v : row) v.re.hi = 1.0;
+  for (auto& v : kc) v.re.hi = 1.0;
+  auto mul = [](Cdd& a, cplx g) { a = cdd_mul(g, a); };
+  // a *= 1 / g for |g| = 1 + e, |e| <= 1e-9: conj(g) (2 - |g|^2) to e^2
+  auto div = [](Cdd& a, cplx g) {
+    a = cdd_mul(std::conj(g), a);
+    const Dd re{g.real(), 0.0}, im{g.imag(), 0.0};
+    const Dd e = dd_add(dd_add(dd_mul_d(re, g.real()), Dd{-1.0, 0.0}), dd_mul_d(im, g.imag()));
+    a = cdd_add(a, cdd_mul(cplx(-e.hi, 0.0), a));
+  };
+  for (int i : B.idx) {
+    const HostOp& op = ops[i];
+    if (op.type == OP_SIGN) {
+      if (P.nsign >= FXP_MAX_SIGNS) return QF_ERR_NOT_SUPPORTED;
+      const uint64_t m = op_bits(op);
+      P.mout[P.nsign] = m & ~win;
+      uint32_t rm = 0;
+      for (int c = 0; c < (1 << G); ++c)
+        if (((uint64_t)P.off[c] & m & win) == (m & win)) rm |= 1u << c;
+      P.rmask[P.nsign++] = (uint16_t)rm;
+      continue;
+    }
+    if (op.type == OP_PHASE) {
+      mul(one[G], op.scalar);
+      P.has_c = 1;
+      continue;
+    }
+    if (op.k == 1) {
+      const int w = wpos(op.gb[0]);
+      Cdd& v = w >= 0 ? one[w] : ratio[G][tpos(op.gb[0])];
+      mul(v, op.diag[1]);
+      if (op.diag[0] != cplx(1, 0)) {
+        div(v, op.diag[0]);
+        mul(one[G], op.diag[0]);
+        P.has_c = 1;
+      }
+      if (w < 0) P.has_c = 1;
+      continue;
+    }
+    int a = op.gb[0], b = op.gb[1];
+    cplx d[2][2] = {{op.diag[0], op.diag[1]}, {op.diag[2], op.diag[3]}};  // [a][b]
+    if (wpos(a) < 0) {
+      std::swap(a, b);
+      std::swap(d[0][1], d[1][0]);
+    }
+    const int wa = wpos(a), wb = wpos(b);
+    if (wa < 0) return QF_ERR_NOT_SUPPORTED;
+    if (wb >= 0) {
+      for (int c = 0; c < (1 << G); ++c) mul(kc[c], d[(c >> wa) & 1][(c >> wb) & 1]);
+      P.has_kc = 1;
+      continue;
+    }
+    const int t = tpos(b);
+    mul(one[wa], d[1][0]);
+    mul(ratio[wa][t], d[1][1]);
+    if (d[0][0] != cplx(1, 0) || d[0][1] != cplx(1, 0)) {
+      P.has_c = 1;
+      mul(one[G], d[0][0]);
+      mul(ratio[G][t], d[0][1]);
+      div(ratio[G][t], d[0][0]);
+      div(one[wa], d[0][0]);
+      mul(ratio[wa][t], d[0][0]);
+      div(ratio[wa][t], d[0][1]);
+    }
+    div(ratio[wa][t], d[1][0]);
+  }
+  auto fixed = [](const Cdd& v) {
+    auto f = [](Dd x) {
+      const double h = std::ldexp(x.hi, FX_F), l = std::ldexp(x.lo, FX_F);
+      const double fh = std::floor(h);
+      return (long long)fh + (long long)std::floor((h - fh) + l + 0.5);
+    };
+    return make_longlong2(f(v.re), f(v.im));
+  };
+  for (int f = 0; f <= G; ++f) {
+    P.one[f] = fixed(one[f]);
+    for (int t = 0; t < n - G; ++t) P.ratio[f][t] = fixed(ratio[f][t]);
+  }
+  for (int c = 0; c < 16; ++c) P.kc[c] = fixed(kc[c]);
+  return QF_OK;
+}
+
+int fx_swap_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, FxSwapParams& P) {
+  std::memset(&P, 0, sizeof(P));
+  P.n = n;
+  int to[64];
+  for (int b = 0; b < n; ++b) to[b] = b;
+  for (int i : B.idx) {
+    to[ops[i].gb[0]] = ops[i].gb[1];
+    to[ops[i].gb[1]] = ops[i].gb[0];
+  }
+  std::vector<int> tile;
+  for (int b = 0; b < n; ++b) {  // the lowest bits with their partners, ten at most
+    if (std::find(tile.begin(), tile.end(), b) != tile.end()) continue;
+    const int need = to[b] == b ? 1 : 2;
+    if ((int)tile.size() + need > FXSW_TILE_BITS) continue;
+    tile.push_back(b);
+    if (need == 2) tile.push_back(to[b]);
+  }
+  std::sort(tile.begin(), tile.end());
+  P.nt = (int)tile.size();
+  for (int j = 0; j < P.nt; ++j) {
+    P.tb[j] = (uint8_t)tile[j];
+    P.lp[j] = (uint8_t)(std::find(tile.begin(), tile.end(), to[tile[j]]) - tile.begin());
+  }
+  for (int b = 0; b < n; ++b)
+    if (to[b] > b && std::find(tile.begin(), tile.end(), b) == tile.end()) {
+      if (P.npair == 16) return QF_ERR_NOT_SUPPORTED;
+      P.pa[P.npair] = (uint8_t)b;
+      P.pb[P.npair++] = (uint8_t)to[b];
+    }
+  return QF_OK;
+}
+
+// The tensor-core plan of one greedy block whose ops all have a fixed-point
+// kernel.  Diagonal gates that reach outside the block's window leave it:
+// those that no later dense gate of the block touches wait in `pending`
+// (which the caller carries to the next block), those that no earlier one
+// touches run before it, and where one sits between two dense gates the
+// block is cut.  Waiting diagonals whose bits all lie in a later window are
+// multiplied into its matrix.
+void plan_tensor_block(const std::vector<HostOp>& ops, int n, const FxBlock& whole, std::vector<int>& pending,
+                       std::vector<FxBlock>& out, int fusion_k) {
+  static thread_local TxParams tp;  // ~5 KiB: kept off the stack
+  auto is_dense = [&](int i) { return ops[i].type == OP_DENSE1 || ops[i].type == OP_DENSE2; };
+  uint64_t win = 0;
+  for (int j = 0; j < whole.G; ++j) win |= uint64_t(1) << whole.order[j];
+  auto leaves = [&](int i) { return ops[i].type == OP_DIAG && (op_bits(ops[i]) & ~win); };
+  size_t at = 0;
+  while (at < whole.idx.size()) {
+    // the segment: up to a dense gate that would pin a diagonal inside it
+    std::vector<int> seg;
+    uint64_t dense = 0, stuck = 0;  // bits of dense gates; of diagonals that follow one on their bits
+    for (; at < whole.idx.size(); ++at) {
+      const int i = whole.idx[at];
+      if (is_dense(i)) {
+        if (op_bits(ops[i]) & stuck) break;
+        dense |= op_bits(ops[i]);
+      } else if (leaves(i) && (op_bits(ops[i]) & dense)) {
+        stuck |= op_bits(ops[i]);
+      }
+      seg.push_back(i);
+    }
+    FxBlock core;
+    core.G = whole.G;
+    for (int j = 0; j < whole.G; ++j) core.order[j] = whole.order[j];
+    // window bits left over: those that let diagonals of the segment, or
+    // waiting ones, into it
+    while (core.G < std::min(fusion_k, FX_G_MAX)) {
+      uint64_t cw = 0;
+      for (int j = 0; j < core.G; ++j) cw |= uint64_t(1) << core.order[j];
+      int count[64] = {0}, best = -1;
+      auto want = [&](int i) {
+        const uint64_t o = op_bits(ops[i]) & ~cw;
+        if (ops[i].type != OP_DIAG || __builtin_popcountll(o) != 1) return;
+        const int b = __builtin_ctzll(o);
+        ++count[b];
+        if (best < 0 || count[b] > count[best]) best = b;
+      };
+      for (int i : seg) want(i);
+      for (int i : pending) want(i);
+      if (best < 0) break;
+      core.order[core.G++] = best;
+    }
+    uint64_t cw = 0;
+    for (int j = 0; j < core.G; ++j) cw |= uint64_t(1) << core.order[j];
+    std::vector<int> wait, post;
+    for (int i : pending) (op_bits(ops[i]) & ~cw || ops[i].type == OP_SIGN ? wait : core.idx).push_back(i);
+    uint64_t seen = 0;
+    for (int i : seg) {
+      const HostOp& op = ops[i];
+      if (is_dense(i)) {
+        seen |= op_bits(op);
+        core.idx.push_back(i);
+      } else if (op.type == OP_DIAG && (op_bits(op) & ~cw)) {
+        // a later dense gate on its bits: it has none before (the segment
+        // would have ended), so it runs first
+        uint64_t later = 0;
+        bool past = false;
+        for (int k : seg) {
+          if (k == i) past = true;
+          else if (past && is_dense(k)) later |= op_bits(ops[k]);
+        }
+        (op_bits(op) & later ? wait : post).push_back(i);
+      } else {
+        core.idx.push_back(i);
+      }
+    }
+    // core.idx holds ops in circuit order behind the absorbed ones
+    emit_phases(ops, wait, dense, out);
+    pending.swap(wait);
+    pending.insert(pending.end(), post.begin(), post.end());
+    if (core.idx.empty()) continue;
+    const bool lone2x2 = core.idx.size() == 1 && ops[core.idx[0]].type == OP_DENSE1;
+    if (!lone2x2 && dense && tx_prepare(n, ops, core, tp, false) == QF_OK) {
+      core.shape = FXB_TENSOR;
+      out.push_back(std::move(core));
+      continue;
+    }
+    // as far as the CUDA-core kernels take it in one pass
+    std::vector<FxBlock> parts = fx_blocks(ops, core.idx, fusion_k, false);
+    for (FxBlock& part : parts) {
+      const bool lone = part.idx.size() == 1 && ops[part.idx[0]].type == OP_DENSE1;
+      if (!lone && tx_prepare(n, ops, part, tp, false) == QF_OK) {
+        part.shape = FXB_TENSOR;
+        out.push_back(std::move(part));
+        continue;
+      }
+      std::vector<FxBlock> one(1, std::move(part));
+      for (FxBlock& b : fx_split_shapes(one, ops)) out.push_back(std::move(b));
+    }
+  }
+}
+
+}  // namespace
+
+// The passes to run.  Blocks the tensor-core pass takes stay whole, the
+// diagonals around them run as phase passes, and the rest is cut into
+// straight-line shapes.
 std::vector<FxBlock> fx_plan_final(std::vector<HostOp>& ops, int n, int& fusion_k) {
   if (!g_fx_tensor || n < 11) return fx_plan(ops, n, fusion_k);
-  std::vector<FxBlock> blocks = fx_plan(ops, n, fusion_k, false, true);
+  fx_merge(ops, n, fusion_k);
+  std::vector<int> all(ops.size());
+  for (size_t i = 0; i < ops.size(); ++i) all[i] = (int)i;
+  std::vector<FxBlock> blocks = fx_blocks(ops, all, fusion_k, true);
   std::vector<FxBlock> out;
+  std::vector<int> pending;  // diagonals not yet applied; all later ops of the plan so far commute with them
   out.reserve(blocks.size());
-  static thread_local TxParams tp;  // ~5 KiB: kept off the stack
+  static thread_local TxParams tp;
+  const uint64_t everything = ~uint64_t(0);
   for (FxBlock& B : blocks) {
-    if (B.wide) {  // a 3- or 4-qubit gate: alone on the tensor cores, else native FP64
-      if (tx_prepare(n, ops, B, tp, false) == QF_OK) B.shape = -2;
-      else B.native = true;
+    if (B.native || B.wide || B.shape == FXB_SWAP) {
+      emit_phases(ops, pending, everything, out);
+      if (B.wide) {  // a 3- or 4-qubit gate: alone on the tensor cores, else native FP64
+        if (tx_prepare(n, ops, B, tp, false) == QF_OK) B.shape = FXB_TENSOR;
+        else B.native = true;
+      }
       out.push_back(std::move(B));
       continue;
     }
-    // a lone 2x2 gate streams faster through the CUDA-core sweep
-    const bool lone2x2 = B.idx.size() == 1 && ops[B.idx[0]].type == OP_DENSE1;
-    if (!lone2x2 && tx_prepare(n, ops, B, tp, false) == QF_OK) {
-      B.shape = -2;
-      out.push_back(std::move(B));
+    bool phases = true;
+    for (int i : B.idx) phases = phases && (phase_op(ops[i]) || ops[i].type == OP_DENSE1 || ops[i].type == OP_DENSE2);
+    if (phases && B.G == 0) {
+      pending.insert(pending.end(), B.idx.begin(), B.idx.end());
+      if (fusion_k == 1) emit_phases(ops, pending, everything, out);
       continue;
     }
-    std::vector<FxBlock> one(1, std::move(B));
-    for (FxBlock& b : fx_split_shapes(one, ops)) out.push_back(std::move(b));
+    if (!phases) {  // a three-qubit diagonal: the interpreted kernels
+      emit_phases(ops, pending, everything, out);
+      std::vector<FxBlock> parts = fx_blocks(ops, B.idx, fusion_k, false);
+      for (FxBlock& part : parts) {
+        if (part.G > 0 && tx_prepare(n, ops, part, tp, false) == QF_OK) {
+          part.shape = FXB_TENSOR;
+          out.push_back(std::move(part));
+          continue;
+        }
+        std::vector<FxBlock> one(1, std::move(part));
+        for (FxBlock& b : fx_split_shapes(one, ops)) out.push_back(std::move(b));
+      }
+      continue;
+    }
+    plan_tensor_block(ops, n, B, pending, out, fusion_k);
   }
+  emit_phases(ops, pending, everything, out);
   return out;
 }
 
@@ -1317,8 +1698,30 @@ int fx_run_ops(const void* in, void* out, int n, std::vector<HostOp>& ops, int f
   static thread_local FxGroupParams gp;  // ~18 KiB: kept off the stack
   static thread_local FxShapeParams sp;
   static thread_local TxParams tp;
+  static thread_local FxPhaseParams pp;
   for (FxBlock& B : blocks) {
     int rc;
+    if (B.shape == FXB_PHASE || B.shape == FXB_SWAP) {
+      LaunchTimer timer(QF_KERNEL_FX_ELEMENTWISE, stream);
+      if (B.shape == FXB_PHASE) {
+        rc = fx_phase_prepare(n, ops, B, pp);
+        if (rc) return rc;
+        pp.in = reinterpret_cast<const double2*>(src);
+        pp.out = reinterpret_cast<double2*>(out);
+        rc = fx_phase_launch(pp, stream);
+      } else {
+        FxSwapParams xp;
+        rc = fx_swap_prepare(n, ops, B, xp);
+        if (rc) return rc;
+        xp.in = reinterpret_cast<const double2*>(src);
+        xp.out = reinterpret_cast<double2*>(out);
+        rc = fx_swap_launch(xp, stream);
+      }
+      if (rc) return rc;
+      ++passes;
+      src = out;
+      continue;
+    }
     switch (fx_block_kernel(ops, B)) {
       case 6: {
         rc = tx_prepare(n, ops, B, tp);
