@@ -417,6 +417,7 @@ __device__ void smem_op(const TileParams& P, const TileOp& op, const Coef* cf,
     }
     default: {  // element-wise ops
       ElemOp eo;
+      eo.real = 0;
       eo.type = op.type;
       eo.k = op.k;
       eo.gb[0] = op.gb[0];
