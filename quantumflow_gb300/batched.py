@@ -58,6 +58,7 @@ class QAOABatch:
         self.count = len(graphs)
         self.ns = np.zeros(self.count, dtype=np.int64)
         self.ps = np.asarray(ps, dtype=np.int64)
+        self._ps_list = ps
         self.nedges = np.zeros(self.count, dtype=np.int64)
         edges_all = []
         for i, g in enumerate(graphs):
@@ -160,12 +161,12 @@ class QAOABatch:
     # ------------------------------------------------------------ angles ---
     def set_angles(self, betas, gammas):
         """Per-instance beta and gamma sequences (lists of length-p arrays)."""
-        host = np.zeros(self.angles.numel())
-        for i in range(self.count):
-            p, a = int(self.ps[i]), int(self.angle_offset[i])
-            host[a:a + p] = np.asarray(betas[i], dtype=np.float64).reshape(p)
-            host[a + p:a + 2 * p] = np.asarray(gammas[i], dtype=np.float64).reshape(p)
-        self.angles.copy_(torch.from_numpy(host))
+        parts = []
+        for i, p in enumerate(self._ps_list):
+            parts.append(np.asarray(betas[i], dtype=np.float64).reshape(p))
+            parts.append(np.asarray(gammas[i], dtype=np.float64).reshape(p))
+        if parts:
+            self.angles.copy_(torch.from_numpy(np.concatenate(parts)))
 
     def get_angles(self):
         host = self.angles.cpu().numpy()
@@ -201,13 +202,13 @@ class QAOABatch:
         """Run once; return (E, dbetas, dgammas) on the host (input order)."""
         self.launch()
         o = self.out.cpu().numpy()
-        es, dbs, dgs = [], [], []
-        for i in range(self.count):
-            p, off = int(self.ps[i]), int(self.out_offset[i])
+        dbs, dgs = [], []
+        off = 0
+        for p in self._ps_list:  # outputs in input order: dgamma, dbeta, <C>
             dgs.append(o[off:off + p].copy())
             dbs.append(o[off + p:off + 2 * p].copy())
-            es.append(o[off + 2 * p])
-        return np.array(es), dbs, dgs
+            off += 2 * p + 1
+        return o[self.out_offset + 2 * self.ps], dbs, dgs
 
     # ------------------------------------------------------------ Adam -----
     def optimizer_reset(self, maxcut=None, target=None):

@@ -157,6 +157,8 @@ class Kraus(Operation):
         """sum_k w_k K_k (.) K_k^dagger as one superoperator."""
         qubits = self.qubits
         N = len(qubits)
+        if self.operators and all(tuple(op.qubits) == qubits for op in self.operators):
+            return Channel(self._superop().reshape([2] * 4 * N), qubits)
         ident = gate_aschannel(Gate(np.eye(2 ** N), qubits=qubits))
         chans = [gate_aschannel(op) @ ident for op in self.operators]
         chans = [c * w for c, w in zip(chans, self.weights)]
@@ -170,6 +172,19 @@ class Kraus(Operation):
         probs /= np.sum(probs)
         pick = np.random.choice(len(res), p=probs)
         return res[pick].normalize()
+
+    def _superop(self) -> np.ndarray:
+        """The superoperator matrix when every operator acts on
+        ``self.qubits``: (ket-out, bra-out) x (ket-in, bra-in) entries
+        sum_k w_k K_k[i, k] conj(K_k)[j, l], the products and the order of
+        the sum those of the general composition."""
+        total = None
+        for op, w in zip(self.operators, self.weights):
+            u = op.asoperator()
+            t = u[:, None, :, None] * u.conj()[None, :, None, :] * w
+            total = t if total is None else total + t
+        d = total.shape[0]
+        return total.reshape(d * d, d * d)
 
     def evolve(self, rho: Density) -> Density:
         """On the GPU as one superoperator pass (equal to the reference's
@@ -217,6 +232,20 @@ class Dephasing(UnitaryMixture):
 
     def __init__(self, prob: float, q0: Qubit) -> None:
         super().__init__([I(q0), Z(q0)], [1 - prob / 2, prob / 2])
+
+
+def narrow_superop(elem):
+    """The superoperator of a channel on one or two qubits that evolves as one
+    pass (its class does not override how), else None."""
+    cls = type(elem)
+    if getattr(cls, "evolve", None) not in (Channel.evolve, Kraus.evolve):
+        return None
+    k = len(elem.qubits)
+    if k > 2:
+        return None
+    if cls.evolve is Channel.evolve:
+        return elem.tensor.reshape(4 ** k, 4 ** k)
+    return elem.aschannel().tensor.reshape(4 ** k, 4 ** k)
 
 
 def join_channels(*channels: Channel) -> Channel:

@@ -5,6 +5,7 @@ the native planner fuses consecutive gates into blocks and sweeps the state
 once per block instead of once per gate (the reference loops
 ``ket = elem.run(ket)`` at quantumflow/circuits.py:97-98).
 """
+import operator
 from typing import Iterable, Iterator
 
 import numpy as np
@@ -23,10 +24,14 @@ __all__ = ["Circuit", "count_operations", "map_gate", "reversal_circuit", "qft_c
 class Circuit(Operation):
     """A sequence of operations (quantumflow/circuits.py:35-138)."""
 
+    _is_circuit = True
+
     def __init__(self, elements: Iterable[Operation] = None) -> None:
         self.elements = list(elements) if elements is not None else []
-        self._pack_key = None
+        self._pack_flat = None  # the gates, qubits and arrays of the last packing
+        self._pack_qubits = None
         self._pack = None
+        self._pack_narrow = False
 
     def add(self, other: "Circuit") -> "Circuit":
         return Circuit(self.elements + other.elements)
@@ -60,7 +65,7 @@ class Circuit(Operation):
         """Flattened gate list (nested circuits expanded)."""
         out = []
         for e in self.elements:
-            if isinstance(e, Circuit):
+            if getattr(e, "_is_circuit", False):
                 out.extend(e.gates())
             else:
                 out.append(e)
@@ -68,14 +73,15 @@ class Circuit(Operation):
 
     def packed(self, qubits: Qubits):
         """(op_k, op_axes, op_mats) arrays of the C ABI for a state on `qubits`."""
-        flat = self.gates()
-        key = (tuple(qubits), tuple(id(g) for g in flat))
-        if key == self._pack_key:
+        return self._packed(self.gates(), tuple(qubits))
+
+    def _packed(self, flat, qubits):
+        if self._is_packed(flat, qubits):
             return self._pack
         index = {q: i for i, q in enumerate(qubits)}
         ks, axes, mats = [], [], []
         for g in flat:
-            if not isinstance(g, Gate):
+            if not getattr(g, "_is_gate", False):
                 raise TypeError(f"{type(g).__name__} cannot run inside a fused circuit")
             ks.append(g.qubit_nb)
             axes.extend(index[q] for q in g.qubits)
@@ -83,8 +89,15 @@ class Circuit(Operation):
         op_k = np.asarray(ks, dtype=np.int32)
         op_axes = np.asarray(axes, dtype=np.int32)
         op_mats = np.ascontiguousarray(np.concatenate(mats) if mats else np.zeros(1))
-        self._pack_key, self._pack = key, (op_k, op_axes, op_mats, len(flat))
+        self._pack_flat, self._pack_qubits = flat, qubits
+        self._pack = (op_k, op_axes, op_mats, len(flat))
         return self._pack
+
+    def _is_packed(self, flat, qubits) -> bool:
+        """Whether the arrays at hand are those of these very gates (held by
+        the packing, so none of them can have been replaced)."""
+        return (self._pack_flat is not None and self._pack_qubits == qubits
+                and len(flat) == len(self._pack_flat) and all(map(operator.is_, flat, self._pack_flat)))
 
     def run(self, ket: State = None, fusion_k: int = None) -> State:
         """Apply the circuit (quantumflow/circuits.py:87-99); default initial
@@ -94,13 +107,18 @@ class Circuit(Operation):
         if fresh:
             ket = zero_state(self.qubits)
         flat = self.gates()
-        if any(not isinstance(g, Gate) or g.qubit_nb > nat.MAX_GATE_QUBITS for g in flat):
+        qubits = tuple(ket.qubits)
+        # (gates packed before, all of them narrow enough, are not looked at again)
+        if not (self._pack_narrow and self._is_packed(flat, qubits)):
+            self._pack_narrow = all(getattr(g, "_is_gate", False) and g.qubit_nb <= nat.MAX_GATE_QUBITS
+                                    for g in flat)
+        if not self._pack_narrow:
             # mixed operations: each run of consecutive gates is one fused
             # launch, other operations (and gates wider than the fused
             # engine takes) run on their own in between
             pending = []
             for elem in flat:
-                if isinstance(elem, Gate) and elem.qubit_nb <= nat.MAX_GATE_QUBITS:
+                if getattr(elem, "_is_gate", False) and elem.qubit_nb <= nat.MAX_GATE_QUBITS:
                     pending.append(elem)
                     continue
                 if pending:
@@ -110,7 +128,7 @@ class Circuit(Operation):
             if pending:
                 ket = Circuit(pending).run(ket, fusion_k)
             return ket
-        op_k, op_axes, op_mats, nops = self.packed(ket.qubits)
+        op_k, op_axes, op_mats, nops = self._packed(flat, qubits)
         src = ket.buffer.compute()
         out = src if (fresh or src is not ket.buffer) else src.empty_like()
         passes = (nat.ctypes.c_int * 1)()
@@ -122,15 +140,24 @@ class Circuit(Operation):
 
     def evolve(self, rho=None):
         """Apply the circuit to a density matrix (quantumflow/circuits.py
-        Circuit.evolve); each run of consecutive gates is one fused launch on
-        the density's ket and bra axes.  Default: |0...0><0...0|."""
+        Circuit.evolve); each run of consecutive gates and one- or two-qubit
+        channels is one fused launch on the density's ket and bra axes.
+        Default: |0...0><0...0|."""
+        from .channels import narrow_superop
         from .densities import evolve_gates
         if rho is None:
             rho = zero_state(self.qubits).asdensity()
+        # channels join the launch where the planner keeps them apart from
+        # the unitary gates (fixed point) or a merged pass costs the same
+        join = rho.dtype == "complex64" or config.C128_ARITHMETIC == "fx"
         pending = []
         for elem in self.gates():
-            if isinstance(elem, Gate):
+            if getattr(elem, "_is_gate", False):
                 pending.append(elem)
+                continue
+            superop = narrow_superop(elem) if join else None
+            if superop is not None:
+                pending.append((superop, elem.qubits))
                 continue
             if pending:
                 rho = evolve_gates(rho, pending)

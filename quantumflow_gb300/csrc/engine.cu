@@ -1757,10 +1757,10 @@ static bool mergeable(const HostOp& op) {
   return false;
 }
 
-static std::vector<cplx> dense_of(const HostOp& op) {
+static CMat dense_of(const HostOp& op) {
   const int G = 1 << op.k;
   if ((int)op.m.size() == G * G) return op.m;
-  std::vector<cplx> m((size_t)G * G, cplx(0, 0));
+  CMat m((size_t)G * G, cplx(0, 0));
   if (op.type == OP_DIAG) {
     for (int r = 0; r < G; ++r) m[r * G + r] = op.diag[r];
   } else if (op.type == OP_SIGN) {
@@ -1772,9 +1772,9 @@ static std::vector<cplx> dense_of(const HostOp& op) {
 }
 
 // the matrix of `op` (k = 1 or 2) acting on the bits `bits` (MSB first, 2 bits)
-static std::vector<cplx> embed2(const HostOp& op, const int bits[2]) {
-  const std::vector<cplx> m = dense_of(op);
-  std::vector<cplx> e(16, cplx(0, 0));
+static CMat embed2(const HostOp& op, const int bits[2]) {
+  const CMat m = dense_of(op);
+  CMat e(16, cplx(0, 0));
   if (op.k == 1) {
     const bool msb = op.gb[0] == bits[0];
     for (int r = 0; r < 4; ++r)
@@ -1792,32 +1792,34 @@ static std::vector<cplx> embed2(const HostOp& op, const int bits[2]) {
   return e;
 }
 
-static std::vector<cplx> matmul_n(const std::vector<cplx>& a, const std::vector<cplx>& b, int G) {
-  std::vector<cplx> c((size_t)G * G, cplx(0, 0));
+static CMat matmul_n(const CMat& a, const CMat& b, int G) {
+  CMat c((size_t)G * G, cplx(0, 0));
   for (int i = 0; i < G; ++i)
     for (int k = 0; k < G; ++k) {
-      const cplx v = a[i * G + k];
-      if (v == cplx(0, 0)) continue;
-      for (int j = 0; j < G; ++j) c[i * G + j] += v * b[k * G + j];
+      const double vr = a[i * G + k].real(), vi = a[i * G + k].imag();
+      if (vr == 0.0 && vi == 0.0) continue;
+      for (int j = 0; j < G; ++j) {  // (std::complex's product tests every result for NaN)
+        const double br = b[k * G + j].real(), bi = b[k * G + j].imag();
+        c[i * G + j] += cplx(vr * br - vi * bi, vr * bi + vi * br);
+      }
     }
   return c;
 }
 
 // rebuild `op` as the gate with matrix m on bits (k = 1 or 2), re-classified
-static void set_matrix(HostOp& op, int k, const int* bits, const std::vector<cplx>& m) {
-  std::vector<double> flat(2 * m.size());
-  for (size_t i = 0; i < m.size(); ++i) {
-    flat[2 * i] = m[i].real();
-    flat[2 * i + 1] = m[i].imag();
-  }
+static void set_matrix(HostOp& op, int k, const int* bits, const CMat& m) {
   HostOp r;
-  classify_op(k, bits, flat.data(), r);
-  op = r;
+  classify_op(k, bits, reinterpret_cast<const double*>(m.data()), r);
+  op = std::move(r);
 }
 
 static bool dense_cost(const HostOp& op) { return op.type == OP_DENSE1 || op.type == OP_DENSE2; }
 
-void merge_ops(std::vector<HostOp>& ops, int n) {
+// `kind` (or null) sorts the gates into kinds that are only merged among
+// themselves: a non-unitary gate would take the unitary ones merged with it
+// from the fixed-point kernels to native FP64.
+void merge_ops(std::vector<HostOp>& ops, int n, int (*kind)(const HostOp&)) {
+  auto alike = [&](const HostOp& a, const HostOp& b) { return kind == nullptr || kind(a) == kind(b); };
   std::vector<HostOp> out;
   std::vector<char> alive;
   std::vector<int> last(n, -1);
@@ -1837,7 +1839,7 @@ void merge_ops(std::vector<HostOp>& ops, int n) {
     if (o.k == 1) {
       const int q = o.gb[0];
       const int t = last[q];
-      if (t >= 0 && alive[t] && mergeable(out[t]) && (dense_cost(out[t]) || out[t].k == 1)) {
+      if (t >= 0 && alive[t] && mergeable(out[t]) && (dense_cost(out[t]) || out[t].k == 1) && alike(out[t], o)) {
         HostOp& d = out[t];
         if (d.k == 1) {
           const int bits[1] = {q};
@@ -1857,15 +1859,15 @@ void merge_ops(std::vector<HostOp>& ops, int n) {
     const int a = o.gb[0], b = o.gb[1];
     const int bits[2] = {a, b};
     const int ta = last[a], tb = last[b];
-    if (ta >= 0 && ta == tb && alive[ta] && mergeable(out[ta]) && out[ta].k == 2) {
+    if (ta >= 0 && ta == tb && alive[ta] && mergeable(out[ta]) && out[ta].k == 2 && alike(out[ta], o)) {
       HostOp& d = out[ta];
       const int dbits[2] = {d.gb[0], d.gb[1]};
       set_matrix(d, 2, dbits, matmul_n(embed2(o, dbits), dense_of(d), 4));
       continue;
     }
-    std::vector<cplx> m = dense_of(o);
+    CMat m = dense_of(o);
     auto pending = [&](int t) {  // a live 1-qubit gate that is the last on its qubit
-      return t >= 0 && alive[t] && mergeable(out[t]) && out[t].k == 1;
+      return t >= 0 && alive[t] && mergeable(out[t]) && out[t].k == 1 && alike(out[t], o);
     };
     const bool pa = pending(ta), pb = pending(tb);
     const bool cheap_a = pa && !dense_cost(out[ta]), cheap_b = pb && !dense_cost(out[tb]);

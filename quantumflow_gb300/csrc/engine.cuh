@@ -1,7 +1,9 @@
 // Host+device interface of the gate engine shared by the .cu files.
 #pragma once
 #include <cstdint>
+#include <algorithm>
 #include <complex>
+#include <initializer_list>
 #include <vector>
 #include <cuda_runtime.h>
 #include "qf_common.cuh"
@@ -119,16 +121,71 @@ struct TileParams {
 };
 
 // A host-side classified op (one gate).
+// A short array of complex numbers: N inline, more on the heap.  Gate lists
+// are planned on every call; with std::vector matrices the allocations were
+// most of the planner's time.
+template <int N>
+class SmallC {
+ public:
+  SmallC() = default;
+  SmallC(size_t n, cplx v) { assign(n, v); }
+  SmallC(std::initializer_list<cplx> l) {
+    grow(l.size());
+    std::copy(l.begin(), l.end(), data());
+  }
+  SmallC(const SmallC& o) { copy(o); }
+  SmallC(SmallC&& o) noexcept { take(o); }
+  SmallC& operator=(const SmallC& o) {
+    if (this != &o) copy(o);
+    return *this;
+  }
+  SmallC& operator=(SmallC&& o) noexcept {
+    if (this != &o) take(o);
+    return *this;
+  }
+  void assign(size_t n, cplx v) {
+    grow(n);
+    std::fill(data(), data() + n, v);
+  }
+  void resize(size_t n) { assign(n, cplx(0, 0)); }
+  size_t size() const { return n_; }
+  cplx* data() { return n_ <= N ? reinterpret_cast<cplx*>(inline_) : heap_.data(); }
+  const cplx* data() const { return n_ <= N ? reinterpret_cast<const cplx*>(inline_) : heap_.data(); }
+  cplx& operator[](size_t i) { return data()[i]; }
+  const cplx& operator[](size_t i) const { return data()[i]; }
+
+ private:
+  void grow(size_t n) {
+    n_ = n;
+    if (n > N) heap_.resize(n);
+  }
+  void copy(const SmallC& o) {
+    grow(o.n_);
+    std::copy(o.data(), o.data() + o.n_, data());
+  }
+  void take(SmallC& o) noexcept {
+    n_ = o.n_;
+    if (n_ > N) heap_ = std::move(o.heap_);
+    else std::copy(o.data(), o.data() + n_, data());
+    o.n_ = 0;
+  }
+  size_t n_ = 0;
+  alignas(16) double inline_[2 * N];
+  std::vector<cplx> heap_;
+};
+using CMat = SmallC<16>;
+
 struct HostOp {
   int k = 0;
   int gb[KMAX_DENSE] = {0, 0, 0, 0, 0};  // global bit positions, matrix MSB first
   uint8_t type = 0;
-  std::vector<cplx> m;        // dense: row-major 2^k x 2^k
-  std::vector<cplx> diag;     // OP_DIAG / OP_MONO phases (per output row)
+  CMat m;                     // dense: row-major 2^k x 2^k
+  SmallC<8> diag;             // OP_DIAG / OP_MONO phases (per output row)
   int perm[8] = {0, 1, 2, 3, 4, 5, 6, 7};
   const uint16_t* cuts = nullptr;  // OP_CUT
   std::vector<cplx> table;         // OP_CUT phase per cut value
   cplx scalar{1.0, 0.0};           // OP_PHASE
+  mutable int8_t fx_kind = 0;      // the fixed-point planner's kind, 0 = not looked up
 };
 
 // Fill one coefficient in the arithmetic of `layout`.
@@ -263,7 +320,7 @@ struct LaunchTimer {
 };
 
 // Consecutive gates multiplied into blocks of at most two qubits (host).
-void merge_ops(std::vector<HostOp>& ops, int n);
+void merge_ops(std::vector<HostOp>& ops, int n, int (*kind)(const HostOp&) = nullptr);
 extern int g_merge_gates;
 
 // Passes of complex128 states in 64-bit integer fixed-point arithmetic

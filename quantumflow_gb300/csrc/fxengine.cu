@@ -575,12 +575,16 @@ bool unit_modulus(cplx c) { return std::abs(std::abs(c) - 1.0) <= FX_UNIT_TOL; }
 
 // the fixed-point kernels take unitary gates only (their overflow bound
 // rests on the group norm being preserved)
-bool unitary(const std::vector<cplx>& m, int G) {
+bool unitary(const CMat& m, int G) {
   for (int i = 0; i < G; ++i)
     for (int j = 0; j < G; ++j) {
-      cplx d(0, 0);
-      for (int k = 0; k < G; ++k) d += m[i * G + k] * std::conj(m[j * G + k]);
-      if (std::abs(d - (i == j ? cplx(1, 0) : cplx(0, 0))) > FX_UNIT_TOL) return false;
+      double dr = i == j ? -1.0 : 0.0, di = 0.0;
+      for (int k = 0; k < G; ++k) {
+        const cplx a = m[i * G + k], b = m[j * G + k];
+        dr += a.real() * b.real() + a.imag() * b.imag();
+        di += a.imag() * b.real() - a.real() * b.imag();
+      }
+      if (!(dr * dr + di * di <= FX_UNIT_TOL * FX_UNIT_TOL)) return false;
     }
   return true;
 }
@@ -588,7 +592,7 @@ bool unitary(const std::vector<cplx>& m, int G) {
 // kinds of op for the fixed-point planner
 enum FxKind { FXK_DENSE = 1, FXK_ELEM = 2, FXK_NATIVE = 3 };
 
-FxKind fx_kind(const HostOp& op) {
+FxKind fx_kind_of(const HostOp& op) {
   switch (op.type) {
     case OP_DENSE1:
     case OP_DENSE2:
@@ -612,6 +616,11 @@ FxKind fx_kind(const HostOp& op) {
   }
 }
 
+FxKind fx_kind(const HostOp& op) {
+  if (op.fx_kind == 0) op.fx_kind = (int8_t)fx_kind_of(op);
+  return (FxKind)op.fx_kind;
+}
+
 int fx_coef_count(const HostOp& op) {
   switch (op.type) {
     case OP_DENSE1: return 4;
@@ -623,10 +632,10 @@ int fx_coef_count(const HostOp& op) {
   return 0;
 }
 
-std::vector<cplx> dense_matrix(const HostOp& op) {
+CMat dense_matrix(const HostOp& op) {
   const int D = 1 << op.k;
   if (op.type != OP_MONO) return op.m;
-  std::vector<cplx> m((size_t)D * D, cplx(0, 0));
+  CMat m((size_t)D * D, cplx(0, 0));
   for (int r = 0; r < D; ++r) m[r * D + op.perm[r]] = op.diag[r];
   return m;
 }
@@ -677,7 +686,8 @@ std::vector<FxBlock> fx_plan(std::vector<HostOp>& ops, int n, int& fusion_k) {
 
 void fx_merge(std::vector<HostOp>& ops, int n, int& fusion_k) {
   if (fusion_k <= 0) fusion_k = FX_G_MAX;
-  if (fusion_k > 1 && g_merge_gates) merge_ops(ops, n);
+  if (fusion_k > 1 && g_merge_gates)
+    merge_ops(ops, n, [](const HostOp& op) { return fx_kind(op) == FXK_NATIVE ? 1 : 0; });
   // generalised permutations on <= 2 qubits with unit-modulus entries run as
   // dense gates here (one code path for the fixed-point passes)
   for (HostOp& op : ops)
@@ -824,7 +834,7 @@ int grid_cap(int64_t items) {
 int launch_fx_single(const void* in, void* out, int n, const HostOp& op, cudaStream_t stream) {
   const double2* src = reinterpret_cast<const double2*>(in);
   double2* dst = reinterpret_cast<double2*>(out);
-  const std::vector<cplx> m = dense_matrix(op);
+  const CMat m = dense_matrix(op);
   if (op.k == 1) {
     FxCoef4 u;
     for (int i = 0; i < 4; ++i) u.c[i] = make_fxc(m[i].real(), m[i].imag());
@@ -913,7 +923,7 @@ int fx_group_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, Fx
     const int need = fx_coef_count(op);
     if (nc + need > FXG_MAX_COEF || no + 3 > FXG_MAX_OPS) return QF_ERR_NOT_SUPPORTED;
     if (fx_kind(op) == FXK_DENSE) {
-      const std::vector<cplx> m = dense_matrix(op);
+      const CMat m = dense_matrix(op);
       if (op.k == 1) {
         swap_to(reg_of(op.gb[0]), G - 1);
         FxGroupOp& g = P.ops[no++];
@@ -1132,17 +1142,91 @@ inline Cdd cdd_mul(cplx g, const Cdd& v) {
           dd_add(dd_mul_d(v.im, g.real()), dd_mul_d(v.re, g.imag()))};
 }
 inline Cdd cdd_add(const Cdd& a, const Cdd& b) { return {dd_add(a.re, b.re), dd_add(a.im, b.im)}; }
-// v * 2^62 of a double-double rounded to the nearest integer, ties away
-// from zero
-inline int64_t dd_fixed62(Dd v) {
-  const double h = std::ldexp(v.hi, 62), l = std::ldexp(v.lo, 62);
-  const double fh = std::floor(h);
-  const double frac = (h - fh) + l;  // h - fh is exact; |l| is below half an ulp of h
-  int64_t r = static_cast<int64_t>(fh);
-  if (frac > 0.5 || (frac == 0.5 && h > 0.0)) ++r;
-  else if (frac < -0.5 || (frac == -0.5 && h < 0.0)) --r;
-  return r;
-}
+// The pass unitary as 2^62 integers.  A gate's entries are rounded to that
+// grid and products are exact in 128 bits, rounded once per gate and entry:
+// k gates err by at most about k 2^-62, below the 2^-59 truncation of every
+// amplitude of the pass.  A product touches only the entries that can be
+// nonzero (rows and columns that agree outside the bits of the gates so far).
+// Three 4x4 gates on a window: 25 -> 10 us of host time a pass, launch included,
+// against double-double products over all entries.
+using i128 = __int128;
+inline int64_t fixed62(double v) { return std::llround(std::ldexp(v, 62)); }
+inline int64_t round62(i128 v) { return static_cast<int64_t>((v + (i128(1) << 61)) >> 62); }
+struct TxUnitary {
+  int64_t re[16][16], im[16][16];
+  uint32_t used = 0;  // window bits of the gates so far
+  void identity() {
+    std::memset(re, 0, sizeof(re));
+    std::memset(im, 0, sizeof(im));
+    for (int c = 0; c < 16; ++c) re[c][c] = int64_t(1) << 62;
+    used = 0;
+  }
+  // f(r, c) for the entries that can be nonzero
+  template <typename F>
+  void entries(F f) {
+    for (int r = 0; r < 16; ++r)
+      for (uint32_t sub = used;; sub = (sub - 1) & used) {
+        f(r, static_cast<int>((r & ~used) | sub));
+        if (sub == 0) break;
+      }
+  }
+  void scale_row_entry(int r, int c, int64_t gr, int64_t gi) {
+    const int64_t ur = re[r][c], ui = im[r][c];
+    re[r][c] = round62(i128(gr) * ur - i128(gi) * ui);
+    im[r][c] = round62(i128(gr) * ui + i128(gi) * ur);
+  }
+  // U <- E U, E the gate m on the window bits jp[0..k) (jp[0] the matrix MSB)
+  void apply(const CMat& m, int k, const int* jp) {
+    const int D = 1 << k;
+    int64_t gr[256], gi[256];
+    for (int e = 0; e < D * D; ++e) {
+      gr[e] = fixed62(m[e].real());
+      gi[e] = fixed62(m[e].imag());
+    }
+    uint32_t om = 0;
+    int spread[16];
+    for (int j = 0; j < k; ++j) om |= 1u << jp[j];
+    for (int x = 0; x < D; ++x) {
+      spread[x] = 0;
+      for (int j = 0; j < k; ++j)
+        if ((x >> (k - 1 - j)) & 1) spread[x] |= 1 << jp[j];
+    }
+    const uint32_t all = used | om;
+    int64_t tr[16][16], ti[16][16];
+    std::memset(tr, 0, sizeof(tr));
+    std::memset(ti, 0, sizeof(ti));
+    for (int base = 0; base < 16; ++base) {
+      if (base & om) continue;
+      for (int x = 0; x < D; ++x) {
+        i128 ar[16], ai[16];
+        std::memset(ar, 0, sizeof(ar));
+        std::memset(ai, 0, sizeof(ai));
+        for (int y = 0; y < D; ++y) {
+          const int64_t er = gr[x * D + y], ei = gi[x * D + y];
+          if (er == 0 && ei == 0) continue;
+          const int row = base | spread[y];
+          for (uint32_t sub = used;; sub = (sub - 1) & used) {
+            const int c = static_cast<int>((row & ~used) | sub);
+            const int64_t ur = re[row][c], ui = im[row][c];
+            ar[c] += i128(er) * ur - i128(ei) * ui;
+            ai[c] += i128(er) * ui + i128(ei) * ur;
+            if (sub == 0) break;
+          }
+        }
+        const int r = base | spread[x];
+        for (uint32_t sub = all;; sub = (sub - 1) & all) {
+          const int c = static_cast<int>((r & ~all) | sub);
+          tr[r][c] = round62(ar[c]);
+          ti[r][c] = round62(ai[c]);
+          if (sub == 0) break;
+        }
+      }
+    }
+    std::memcpy(re, tr, sizeof(re));
+    std::memcpy(im, ti, sizeof(im));
+    used = all;
+  }
+};
 
 // Fill the tensor-core pass of block B (dense unitary gates, unit-modulus
 // diagonals and phases on its window, sign ops), or return
@@ -1152,8 +1236,7 @@ inline int64_t dd_fixed62(Dd v) {
 // the window is moved to the inputs when no earlier dense gate of the block
 // touches its window bits, else to the outputs when no later one does.
 // With `matrix` false only the structure is checked (the planner's test);
-// with it, U is multiplied up in double-double from the gates in block
-// order and rounded to the 2^-62 integers of the kernel.
+// with it, U is multiplied up from the gates in block order (TxUnitary).
 int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams& P, bool matrix = true) {
   if (B.native || B.G < 1 || B.G > 4 || n < 11) return QF_ERR_NOT_SUPPORTED;
   auto dense_op = [](const HostOp& op) {
@@ -1179,13 +1262,8 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
       if ((c >> j) & 1) o |= int64_t(1) << wb[j];
     P.off[c] = o;
   }
-  std::vector<Cdd> U, T;
-  bool identity = true;  // U is still the identity (the first dense gate is copied, not multiplied)
-  if (matrix) {
-    U.assign(256, Cdd());
-    T.assign(256, Cdd());
-    for (int c = 0; c < 16; ++c) U[c * 16 + c].re.hi = 1.0;
-  }
+  static thread_local TxUnitary U;
+  if (matrix) U.identity();
   // window bits each dense op of the block touches, for the sign placement
   std::vector<int> dense_pos;
   std::vector<uint32_t> dense_bits;
@@ -1208,56 +1286,13 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
         if (jp[j] < 0) return QF_ERR_NOT_SUPPORTED;
       }
       if (!matrix) continue;
-      const int D = 1 << op.k;
-      const std::vector<cplx> gm = dense_matrix(op);
-      uint32_t om = 0;
-      for (int j = 0; j < op.k; ++j) om |= 1u << jp[j];
-      auto local = [&](int c) {  // the gate's matrix index of window index c (gate qubit 0 = MSB)
-        int r = 0;
-        for (int j = 0; j < op.k; ++j) r = (r << 1) | ((c >> jp[j]) & 1);
-        return r;
-      };
-      auto spread = [&](int r, int m) {  // window index r with the gate's bits set to m
-        int cm = r & ~static_cast<int>(om);
-        for (int j = 0; j < op.k; ++j)
-          if ((m >> (op.k - 1 - j)) & 1) cm |= 1 << jp[j];
-        return cm;
-      };
-      if (identity) {  // U = E: the gate embedded in the window
-        for (int r = 0; r < 16; ++r)
-          for (int c = 0; c < 16; ++c) {
-            Cdd v;
-            if ((r & ~static_cast<int>(om)) == (c & ~static_cast<int>(om))) {
-              const cplx g = gm[local(r) * D + local(c)];
-              v.re.hi = g.real();
-              v.im.hi = g.imag();
-            }
-            U[r * 16 + c] = v;
-          }
-        identity = false;
-        continue;
-      }
-      // T = E U
-      for (int r = 0; r < 16; ++r) {
-        const int lr = local(r);
-        for (int c = 0; c < 16; ++c) {
-          Cdd acc;
-          for (int m = 0; m < D; ++m) {
-            const cplx g = gm[lr * D + m];
-            const Cdd& u = U[spread(r, m) * 16 + c];
-            if ((g.real() == 0.0 && g.imag() == 0.0) || cdd_zero(u)) continue;
-            acc = cdd_add(acc, cdd_mul(g, u));
-          }
-          T[r * 16 + c] = acc;
-        }
-      }
-      U.swap(T);
+      U.apply(dense_matrix(op), op.k, jp);
       continue;
     }
     if (op.type == OP_PHASE) {
       if (!matrix) continue;
-      for (Cdd& v : U) v = cdd_mul(op.scalar, v);
-      identity = false;
+      const int64_t gr = fixed62(op.scalar.real()), gi = fixed62(op.scalar.imag());
+      U.entries([&](int r, int c) { U.scale_row_entry(r, c, gr, gi); });
       continue;
     }
     if (op.type == OP_DIAG) {
@@ -1267,12 +1302,16 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
         if (jp[j] < 0) return QF_ERR_NOT_SUPPORTED;
       }
       if (!matrix) continue;
-      for (int r = 0; r < 16; ++r) {
+      int64_t gr[8], gi[8];
+      for (int e = 0; e < (1 << op.k); ++e) {
+        gr[e] = fixed62(op.diag[e].real());
+        gi[e] = fixed62(op.diag[e].imag());
+      }
+      U.entries([&](int r, int c) {
         int e = 0;
         for (int j = 0; j < op.k; ++j) e = (e << 1) | ((r >> jp[j]) & 1);
-        for (int c = 0; c < 16; ++c) U[r * 16 + c] = cdd_mul(op.diag[e], U[r * 16 + c]);
-      }
-      identity = false;
+        U.scale_row_entry(r, c, gr[e], gi[e]);
+      });
       continue;
     }
     if (op.type != OP_SIGN) return QF_ERR_NOT_SUPPORTED;
@@ -1288,10 +1327,12 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
       if ((c & jm) == jm) rm |= 1u << c;
     if (mo == 0) {  // inside the window: a diagonal of U
       if (!matrix) continue;
-      for (int r = 0; r < 16; ++r)
-        if ((rm >> r) & 1)
-          for (int c = 0; c < 16; ++c) U[r * 16 + c] = {dd_neg(U[r * 16 + c].re), dd_neg(U[r * 16 + c].im)};
-      identity = false;
+      U.entries([&](int r, int c) {
+        if ((rm >> r) & 1) {
+          U.re[r][c] = -U.re[r][c];
+          U.im[r][c] = -U.im[r][c];
+        }
+      });
       continue;
     }
     bool before = false, after = false;
@@ -1313,14 +1354,14 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
     }
   }
   if (!matrix) return QF_OK;
+  // unit rows of a product of gates unitary to 1e-9: well inside the
+  // digits' bounds (|G| < 2^62.9 keeps G + bias below 2^64)
+  constexpr int64_t LIM = (int64_t(1) << 62) + (int64_t(1) << 42);
   for (int r = 0; r < 16; ++r)
     for (int c = 0; c < 16; ++c) {
-      const Cdd& v = U[r * 16 + c];
-      // unit rows of a product of gates unitary to 1e-9: well inside the
-      // digits' bounds (|G| < 2^62.9 keeps G + bias below 2^64)
-      if (std::abs(v.re.hi) > 1.0 + 1e-6 || std::abs(v.im.hi) > 1.0 + 1e-6) return QF_ERR_NOT_SUPPORTED;
-      P.g[r][c][0] = dd_fixed62(v.re);
-      P.g[r][c][1] = dd_fixed62(v.im);
+      if (std::abs(U.re[r][c]) > LIM || std::abs(U.im[r][c]) > LIM) return QF_ERR_NOT_SUPPORTED;
+      P.g[r][c][0] = U.re[r][c];
+      P.g[r][c][1] = U.im[r][c];
     }
   return QF_OK;
 }

@@ -119,10 +119,18 @@ class Density(State):
 # -------------------------------------------------------------- evolution --
 def evolve_gates(rho: Density, gates) -> Density:
     """Apply gates to rho: U on the ket axes and conj(U) on the bra axes of
-    every gate, as one fused circuit launch on the 2N-qubit buffer."""
+    every gate, as one fused circuit launch on the 2N-qubit buffer.  Elements
+    may also be (superoperator, qubits) pairs of at most two qubits."""
     N = rho.qubit_nb
     ks, axes, mats = [], [], []
     for g in gates:
+        if isinstance(g, tuple):
+            superop, qubits = g
+            idx = [rho.qubits.index(q) for q in qubits]
+            ks.append(2 * len(idx))
+            axes += idx + [N + i for i in idx]
+            mats.append(np.ascontiguousarray(superop, dtype=np.complex128).view(np.float64).reshape(-1))
+            continue
         idx = [rho.qubits.index(q) for q in g.qubits]
         u = np.ascontiguousarray(g.asoperator(), dtype=np.complex128)
         ks += [len(idx), len(idx)]

@@ -23,6 +23,10 @@ class Operation(ABC):
     """An operation on a qubit state (quantumflow/ops.py:35-88)."""
 
     _qubits: Qubits = ()
+    # what a circuit asks of every element of every run; a class attribute
+    # because isinstance on an abstract class costs ten times the lookup
+    _is_gate = False
+    _is_circuit = False
 
     @property
     def qubits(self) -> Qubits:
@@ -62,6 +66,8 @@ class Operation(ABC):
 
 class Gate(Operation):
     """A quantum logic gate (quantumflow/ops.py:91-262)."""
+
+    _is_gate = True
 
     def __init__(self, tensor: Any, qubits: Qubits = None, params: Dict[str, float] = None,
                  name: str = None) -> None:
