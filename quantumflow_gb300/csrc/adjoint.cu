@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "qtile.cuh"
 #include "state.cuh"
 
 namespace qf {
@@ -500,6 +501,8 @@ __global__ void k_rows_sum(const double* rows, int nrows, int nslots, double* ou
 void qaoa_layer_ops(int n, const uint16_t* cuts, int nedges, double beta, double gamma,
                     const double* node_theta, std::vector<HostOp>& ops);
 
+extern int g_force_smem_tile;
+extern int g_warp_rb_override;
 int g_adjoint_smem_only = 0;  // qf_set_tile_kernel(1): shared-memory adjoint kernel only
 
 int adj_grid(int n, int layout) {
@@ -510,8 +513,6 @@ int adj_grid(int n, int layout) {
   if (g > ntiles) g = (int)ntiles;
   return (int)g;
 }
-
-extern int g_warp_rb_override;
 
 // register bits of k_adjw: 2 or 3 for FP64/float-float, 3 or 4 for complex64
 int adjw_rb(int layout) {
@@ -529,11 +530,38 @@ int adjw_grid(int n, int layout) {
   return (int)(g < cap ? g : cap);
 }
 
+// bytes for lambda and `rows` rows of gradient partial sums
+static size_t grad_bytes(int n, int p, int layout, size_t rows) {
+  return (size_t(1) << n) * elem_bytes(layout) + rows * (2 * p + 1) * sizeof(double) + 512;
+}
+// the least workspace qaoa_grad takes (the warp-tile and shared-memory sweeps)
+size_t qaoa_grad_min_bytes(int n, int p, int layout) {
+  return grad_bytes(n, p, layout, std::max(adj_grid(n, layout), adjw_grid(n, layout)));
+}
 size_t qaoa_grad_workspace_bytes(int n, int p, int layout) {
-  const size_t amps = size_t(1) << n;
+  return std::max(qaoa_grad_min_bytes(n, p, layout), grad_bytes(n, p, layout, qtile_grad_rows(n, layout)));
+}
+// Forward state and gradient on wide tiles, or QF_ERR_NOT_SUPPORTED when the
+// case, the settings or a workspace sized for the other sweeps do not allow it.
+int qaoa_wide_grad(void* psi, int n, int layout, const uint16_t* cuts, int nedges, int p, const double* beta,
+                   const double* gamma, const double* node_theta, int fusion_k, double* out, void* ws,
+                   size_t ws_bytes, cudaStream_t stream) {
   const int nslots = 2 * p + 1;
-  const int rows = std::max(adj_grid(n, layout), adjw_grid(n, layout));
-  return amps * elem_bytes(layout) + (size_t)rows * nslots * sizeof(double) + 512;
+  if (fusion_k != 0 || g_force_smem_tile || g_adjoint_smem_only || g_warp_rb_override != 0 ||
+      !qtile_fits(n, layout, nedges, p, node_theta) || nslots > ADJ_MAX_SLOTS)
+    return QF_ERR_NOT_SUPPORTED;
+  const size_t nrows = qtile_grad_rows(n, layout);
+  if (ws_bytes < grad_bytes(n, p, layout, nrows)) return QF_ERR_NOT_SUPPORTED;
+  const size_t amps = size_t(1) << n;
+  double* rows = reinterpret_cast<double*>(static_cast<char*>(ws) + ((amps * elem_bytes(layout) + 255) & ~size_t(255)));
+  int rc = check_cuda(cudaMemsetAsync(rows, 0, nrows * nslots * sizeof(double), stream));
+  if (rc) return rc;
+  rc = qtile_state(psi, n, cuts, nedges, p, beta, gamma, true, stream);
+  if (rc) return rc;
+  rc = qtile_grad(psi, ws, n, cuts, nedges, p, beta, gamma, rows, nslots, stream);
+  if (rc) return rc;
+  k_rows_sum<<<nslots, 32, 0, stream>>>(rows, (int)nrows, nslots, out);
+  return check_cuda(cudaGetLastError());
 }
 
 template <int LAY, int RB>

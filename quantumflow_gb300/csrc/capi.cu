@@ -25,6 +25,10 @@ int apply_dense_gate(const void* in, void* out, int n, int layout, int k, const 
 int qaoa_state(void* psi, int n, int layout, const uint16_t* cuts, int nedges, int p, const double* beta,
                const double* gamma, const double* node_theta, int fusion_k, cudaStream_t stream);
 size_t qaoa_grad_workspace_bytes(int n, int p, int layout);
+size_t qaoa_grad_min_bytes(int n, int p, int layout);
+int qaoa_wide_grad(void* psi, int n, int layout, const uint16_t* cuts, int nedges, int p, const double* beta,
+                   const double* gamma, const double* node_theta, int fusion_k, double* out, void* ws,
+                   size_t ws_bytes, cudaStream_t stream);
 size_t batch_workspace_bytes(int max_n, int layout, int ctas);
 int batch_qaoa(const qf_batch_instance* inst, int ninst, int nlarge, const uint8_t* edges, const double* angles,
                double* out, int layout, int max_n, int ts, int ctas, void* ws, size_t ws_bytes,
@@ -379,10 +383,13 @@ int qf_qaoa_expectation_grad(void* psi, int n, int layout, const uint16_t* cuts,
   if (p > 0 && (beta == nullptr || gamma == nullptr)) return QF_ERR_INVALID_ARGUMENT;
   if (nedges + 1 > 1024 || 2 * p + 1 > 64) return QF_ERR_TOO_LARGE;
   layout = st(layout);
-  rc = check_ws(workspace, workspace_bytes, qaoa_grad_workspace_bytes(n, p, layout));
+  rc = check_ws(workspace, workspace_bytes, qaoa_grad_min_bytes(n, p, layout));
   if (rc) return rc;
   if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return QF_ERR_ALIGNMENT;
   cudaStream_t s = as_stream(stream);
+  rc = qaoa_wide_grad(psi, n, layout, cuts, nedges, p, beta, gamma, node_theta, fusion_k, out, workspace,
+                      workspace_bytes, s);
+  if (rc != QF_ERR_NOT_SUPPORTED) return rc;
   rc = qaoa_state(psi, n, layout, cuts, nedges, p, beta, gamma, node_theta, fusion_k, s);
   if (rc) return rc;
   return qaoa_grad(psi, n, layout, cuts, nedges, p, beta, gamma, node_theta, out, workspace, s);

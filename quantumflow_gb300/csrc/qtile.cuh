@@ -1,0 +1,17 @@
+// QAOA on wide tiles (qtile.cu): forward state and adjoint gradient of
+// float-float states.
+#pragma once
+#include <cstddef>
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace qf {
+
+bool qtile_fits(int n, int layout, int nedges, int p, const double* node_theta);
+size_t qtile_grad_rows(int n, int layout);
+int qtile_state(void* psi, int n, const uint16_t* cuts, int nedges, int p, const double* beta, const double* gamma,
+                bool keep_phi, cudaStream_t stream);
+int qtile_grad(void* psi, void* lam, int n, const uint16_t* cuts, int nedges, int p, const double* beta,
+               const double* gamma, double* rows, int nslots, cudaStream_t stream);
+
+}  // namespace qf
