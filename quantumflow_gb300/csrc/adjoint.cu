@@ -712,9 +712,13 @@ int qaoa_grad(void* psi, int n, int layout, const uint16_t* cuts, int nedges, in
   if (wgrid > 0 && p > 0 && wfits && !g_adjoint_smem_only) {
     int rc = check_cuda(cudaMemsetAsync(rows, 0, (size_t)wgrid * nslots * sizeof(double), stream));
     if (rc) return rc;
-    rc = qaoa_grad_warp(psi, n, layout, cuts, nedges, p, beta, gamma, node_theta, lam, rows, nslots, stream);
+    int nrows = wgrid;
+    if (g_warp_rb_override == 0 && qpair_fits(n, layout, nedges, p, node_theta))
+      rc = qpair_grad(psi, lam, n, cuts, nedges, p, beta, gamma, rows, nslots, &nrows, stream);
+    else
+      rc = qaoa_grad_warp(psi, n, layout, cuts, nedges, p, beta, gamma, node_theta, lam, rows, nslots, stream);
     if (rc) return rc;
-    k_rows_sum<<<nslots, 32, 0, stream>>>(rows, wgrid, nslots, out);
+    k_rows_sum<<<nslots, 32, 0, stream>>>(rows, nrows, nslots, out);
     return check_cuda(cudaGetLastError());
   }
   const int grid = adj_grid(n, layout);

@@ -303,6 +303,8 @@ static int qaoa_state_warp(void* psi, int n, int layout, const uint16_t* cuts, i
 int qaoa_state(void* psi, int n, int layout, const uint16_t* cuts, int nedges, int p, const double* beta,
                const double* gamma, const double* node_theta, int fusion_k, cudaStream_t stream) {
   const int RB = qw_rb(layout);
+  if (fusion_k == 0 && !g_force_smem_tile && g_warp_rb_override == 0 && qpair_fits(n, layout, nedges, p, node_theta))
+    return qpair_state(psi, n, cuts, nedges, p, beta, gamma, stream);
   if (fusion_k == 0 && !g_force_smem_tile && g_warp_rb_override == 0 && qtile_fits(n, layout, nedges, p, node_theta))
     return qtile_state(psi, n, cuts, nedges, p, beta, gamma, false, stream);
   if (p > 0 && fusion_k == 0 && !g_force_smem_tile && n >= 5 + RB && nedges + 1 + 2 * n <= QW_MAX_COEF)

@@ -14,4 +14,12 @@ int qtile_state(void* psi, int n, const uint16_t* cuts, int nedges, int p, const
 int qtile_grad(void* psi, void* lam, int n, const uint16_t* cuts, int nedges, int p, const double* beta,
                const double* gamma, double* rows, int nslots, cudaStream_t stream);
 
+// Two register groups a pass (qpair.cu): one complex64 instance.  The number
+// of rows of partial sums is at most that of the warp-tile sweep.
+bool qpair_fits(int n, int layout, int nedges, int p, const double* node_theta);
+int qpair_state(void* psi, int n, const uint16_t* cuts, int nedges, int p, const double* beta, const double* gamma,
+                cudaStream_t stream);
+int qpair_grad(void* psi, void* lam, int n, const uint16_t* cuts, int nedges, int p, const double* beta,
+               const double* gamma, double* rows, int nslots, int* nrows, cudaStream_t stream);
+
 }  // namespace qf
