@@ -3,7 +3,7 @@
 //
 // Reference semantics: quantumflow/qaoa.py:22-64 and
 // examples/qaoa_maxcut.py:56-64, as in qaoa.cu and adjoint.cu, whose
-// warp-tile passes these replace from 14 qubits on: the same operations in
+// warp-tile passes these replace from 13 qubits on: the same operations in
 // the same order, half of the passes over the state.
 // Bound: HBM (adjoint passes, 106 us at n = 24 of 80 at the copy rate); the
 // forward passes, 69 us of 40, FP32 issue and shuffles at the layer

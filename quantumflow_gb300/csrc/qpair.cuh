@@ -89,8 +89,9 @@ inline PairPass pair_pass(int n, int RB, const PairGroups& g, int first, int sec
   for (int j = 0; j < 2 * RB; ++j) P.s[j] = (uint8_t)all[j];
   return P;
 }
-// smallest n of the two-group passes: a whole tile, and at least two runs
-inline int pair_min_qubits(int RB) { return 5 + 2 * RB + 1; }
+// smallest n of the forward passes (a whole tile); the adjoint ones want two
+// runs of groups, one qubit more
+inline int pair_min_qubits(int RB) { return 5 + 2 * RB; }
 
 // forward passes: |+>^n and p layers
 inline std::vector<PairPass> pair_fwd_passes(int n, int p, int RB) {
@@ -106,6 +107,12 @@ inline std::vector<PairPass> pair_fwd_passes(int n, int p, int RB) {
   PairPass f = make(0, false);  // layer 0 starts upwards: its first group is Y
   f.init = f.cost = f.hasB = 1;
   out.push_back(f);
+  for (int l = 1; m == 1 && l < p; ++l) {  // the tile is the state: a pass per layer
+    PairPass a = make(0, (l & 1) != 0);
+    a.cost = a.hasB = 1;
+    a.layerB = (int16_t)l;
+    out.push_back(a);
+  }
   for (int l = 0; l < p; ++l)
     for (int k = 1; k < m; ++k) {
       const bool up = (l & 1) == 0;

@@ -5,7 +5,10 @@
 // the pass sequences of the single-instance warp-tile kernels (qaoa.cu
 // k_qaoaw, adjoint.cu k_adjw): warp sub-tiles of 32 lanes x 2^RB registers
 // prefetched through a per-warp async-copy ring, layer boundaries merged into
-// one pass.  Wave w launches the w-th pass of every instance that has
+// one pass.  Instances of at least a two-group tile (complex64 13 qubits,
+// float-float 11) take two register groups a pass (qpair.cuh: the same
+// operations in the same order, a third to a half of the passes).  200 graphs
+// of 8 to 18 qubits, complex64: 2295 -> 1545 us of kernels an evaluation.  Wave w launches the w-th pass of every instance that has
 // one -- forward items in one launch, adjoint items in another -- so one
 // launch covers all instances and the launch count is the longest
 // instance's pass count, whatever the batch size.  Every launch reads its
@@ -22,6 +25,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "qpair.cuh"
 #include "state.cuh"
 
 namespace qf {
@@ -451,6 +455,86 @@ __global__ void __launch_bounds__(256) k_wave_adj(const WvAdj* items, int nitems
   }
 }
 
+// ------------------------------------------- two register groups a pass ----
+// A block takes a run of tiles of one item.
+constexpr int WP_TILES_FWD = 2, WP_TILES_ADJ = 4;
+
+// this block's item and instance, and the cut table of `layer` in smem
+template <bool ADJ>
+QF_D bool wp_begin(const PairPass* items, int nitems, const WvInst* inst, const Coef* tab, const int32_t* skip,
+                   Coef* scut, PairPass& F, WvInst& I) {
+  if (threadIdx.x == 0) {
+    F = items[wv_find(items, nitems)];
+    I = inst[F.inst];
+  }
+  __syncthreads();
+  if (skip != nullptr && skip[F.inst] != 0) return false;
+  const int E1 = I.nedges + 1;
+  const Coef* t = tab + I.tab + 3 * I.p + (ADJ ? (int64_t)I.p * E1 + (int64_t)F.layerA * E1 : (int64_t)F.layerB * E1);
+  if (F.cost)
+    for (int j = threadIdx.x; j < E1; j += blockDim.x) scut[j] = t[j];
+  __syncthreads();
+  return true;
+}
+
+template <int LAY, int RB>
+__global__ void __launch_bounds__(PairShape<LAY, RB>::NT) k_wave_pair_fwd(const PairPass* items, int nitems,
+                                                                          const WvInst* inst, void* states,
+                                                                          const uint16_t* cuts, const Coef* tab,
+                                                                          int cutb, const int32_t* skip) {
+  using E = typename Types<LAY>::E;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ PairPass F;
+  __shared__ WvInst I;
+  Coef* scut = reinterpret_cast<Coef*>(smem_raw);
+  if (!wp_begin<false>(items, nitems, inst, tab, skip, scut, F, I)) return;
+  const Coef* t = tab + I.tab;
+  E* tag = nullptr;
+  const E amp0 = coef_e(wv_coef<LAY>(1.0 / sqrt((double)(int64_t(1) << I.n)), 0.0), tag);
+  const uint32_t first = (blockIdx.x - F.block_begin) * WP_TILES_FWD, all = 1u << (I.n - 5 - 2 * RB);
+  const Coef ac = t[3 * F.layerA], as = t[3 * F.layerA + 1], bc = t[3 * F.layerB], bs = t[3 * F.layerB + 1];
+  pair_forward<LAY, RB>(F, reinterpret_cast<E*>(states) + I.psi, cuts + I.cuts, scut, I.nedges + 1, amp0, ac, as, bc,
+                        bs, first, 1u, min(first + WP_TILES_FWD, all), smem_raw + cutb);
+}
+
+template <int LAY, int RB>
+__global__ void __launch_bounds__(PairShape<LAY, RB>::NT) k_wave_pair_adj(const PairPass* items, int nitems,
+                                                                          const WvInst* inst, void* states,
+                                                                          const uint16_t* cuts, const Coef* tab,
+                                                                          double* partials, int cutb,
+                                                                          const int32_t* skip) {
+  using E = typename Types<LAY>::E;
+  constexpr int NW = 1 << RB;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ PairPass F;
+  __shared__ WvInst I;
+  __shared__ double red[NW][4];
+  Coef* scut = reinterpret_cast<Coef*>(smem_raw);
+  if (!wp_begin<true>(items, nitems, inst, tab, skip, scut, F, I)) return;
+  const Coef* t = tab + I.tab;
+  const int lb = F.layerB > 0 ? F.layerB : 0;
+  // RX(-beta) = [[c, i s], [i s, c]]: entries (c, +sin) of the tables
+  const Coef ac = t[3 * F.layerA], as = t[3 * F.layerA + 2], bc = t[3 * lb], bs = t[3 * lb + 2];
+  const uint32_t first = (blockIdx.x - F.block_begin) * WP_TILES_ADJ, all = 1u << (I.n - 5 - 2 * RB);
+  E* psi = reinterpret_cast<E*>(states);
+  PairSums S{};
+  pair_adjoint<LAY, RB, LAY == C64>(F, psi + I.psi, psi + I.lam, cuts + I.cuts, scut, I.nedges + 1,
+                                    0.5f * (float)I.nedges, ac, as, bc, bs, first, 1u,
+                                    min(first + WP_TILES_ADJ, all), smem_raw + cutb, S);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double v[4] = {warp_sum((double)S.a.s + (double)S.a.e), warp_sum((double)S.cut.s + (double)S.cut.e),
+                       warp_sum((double)S.e.s + (double)S.e.e), warp_sum((double)S.b.s + (double)S.b.e)};
+  if (lane == 0)
+    for (int k = 0; k < 4; ++k) red[warp][k] = v[k];
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double sum = 0.0;
+    for (int w = 0; w < NW; ++w) sum += red[w][threadIdx.x];
+    if (threadIdx.x == 1) sum *= -2.0;
+    partials[(int64_t)(F.prow + (blockIdx.x - F.block_begin)) * 4 + threadIdx.x] = sum;
+  }
+}
+
 // out[o] = sum of its segments, in order (one warp per output)
 __global__ void k_wave_reduce(const int32_t* seg_begin, const WvSeg* segs, int nout_total, const int32_t* out_index,
                               const double* partials, double* out) {
@@ -470,17 +554,19 @@ __global__ void k_wave_reduce(const int32_t* seg_begin, const WvSeg* segs, int n
 // ------------------------------------------------------------ host plan ----
 struct WvPlanHeader {
   int32_t magic, layout, rbf, rba;
-  int32_t ninst, nwaves, nfwd, nadj, nsegs, nout;
+  int32_t ninst, nwaves, nfwd, nadj, npfwd, npadj, nsegs, nout;
   int64_t state_elems, cut_elems, tab_coefs, prows;
   // device byte offsets inside the workspace
-  int64_t off_inst, off_fwd, off_adj, off_segbeg, off_segs, off_outidx, off_tab, off_part, off_cuts, off_states;
+  int64_t off_inst, off_fwd, off_adj, off_pfwd, off_padj, off_segbeg, off_segs, off_outidx, off_tab, off_part, off_cuts, off_states;
   int64_t device_bytes;
 };
 struct WvWave {
   int32_t fwd_begin, fwd_count, fwd_blocks;
   int32_t adj_begin, adj_count, adj_blocks;
+  int32_t pfwd_begin, pfwd_count, pfwd_blocks;  // two register groups a pass
+  int32_t padj_begin, padj_count, padj_blocks;
 };
-constexpr int32_t WV_MAGIC = 0x51465756;
+constexpr int32_t WV_MAGIC = 0x51465757;  // the version of this layout
 
 static int wv_rb_fwd(int layout) { return layout == C64 ? 4 : 3; }
 static int wv_rb_adj(int layout) { return layout == C64 ? 3 : 2; }
@@ -494,6 +580,7 @@ struct PlanBuild {
   std::vector<WvInst> inst;
   std::vector<WvFwd> fwd;
   std::vector<WvAdj> adj;
+  std::vector<PairPass> pfwd, padj;
   std::vector<WvWave> waves;
   std::vector<int32_t> segbeg, outidx;
   std::vector<WvSeg> segs;
@@ -602,7 +689,14 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
   P.h.ninst = ninst;
   std::vector<std::vector<WvFwd>> fw(ninst);
   std::vector<std::vector<WvAdj>> ad(ninst);
+  std::vector<std::vector<PairPass>> pf(ninst), pa(ninst);  // instead of fw and ad, for tiles of two groups
   std::vector<std::vector<std::array<int, 4>>> sl(ninst);
+  auto pairs = [&](int n) { return n <= 31 && n >= std::max(pair_min_qubits(RBf), pair_min_qubits(RBa) + 1); };
+  // blocks of one adjoint pass
+  auto adj_blocks = [&](int n) {
+    const int64_t per = pairs(n) ? WP_TILES_ADJ : WV_SUBS_PER_BLOCK;
+    return (int32_t)(((int64_t(1) << (n - 5 - (pairs(n) ? 2 : 1) * RBa)) + per - 1) / per);
+  };
   int64_t st = 0, ct = 0, tb = 0;
   int nw = 0;
   for (int i = 0; i < ninst; ++i) {
@@ -626,9 +720,16 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
     w.tab = tb;
     tb += wv_tab_size(q.p, q.nedges);
     P.inst.push_back(w);
-    wv_fwd_passes(q.n, q.p, RBf, fw[i]);
-    wv_adj_passes(q.n, q.p, RBa, ad[i], sl[i]);
-    nw = std::max(nw, (int)(fw[i].size() + ad[i].size()));
+    if (pairs(q.n)) {
+      pf[i] = pair_fwd_passes(q.n, q.p, RBf);
+      pa[i] = pair_adj_passes(q.n, q.p, RBa);
+      for (const PairPass& a : pa[i])
+        sl[i].push_back({q.p + a.layerA, a.cost ? a.layerA : -1, a.init ? 2 * q.p : -1, a.hasB ? q.p + a.layerB : -1});
+    } else {
+      wv_fwd_passes(q.n, q.p, RBf, fw[i]);
+      wv_adj_passes(q.n, q.p, RBa, ad[i], sl[i]);
+    }
+    nw = std::max(nw, (int)(fw[i].size() + ad[i].size() + pf[i].size() + pa[i].size()));
   }
   // waves: pass w of every instance; adjoint blocks get consecutive rows
   int64_t prow = 0;
@@ -637,11 +738,28 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
     WvWave wave{};
     wave.fwd_begin = (int32_t)P.fwd.size();
     wave.adj_begin = (int32_t)P.adj.size();
-    int32_t fb = 0, ab = 0;
+    wave.pfwd_begin = (int32_t)P.pfwd.size();
+    wave.padj_begin = (int32_t)P.padj.size();
+    int32_t fb = 0, ab = 0, pfb = 0, pab = 0;
     for (int i = 0; i < ninst; ++i) {
-      const int nf = (int)fw[i].size();
+      const int nf = (int)fw[i].size(), npf = (int)pf[i].size();
       const int n = P.inst[i].n;
-      if (w < nf) {
+      if (w < npf) {
+        PairPass f = pf[i][w];
+        f.inst = i;
+        f.block_begin = pfb;
+        pfb += (int32_t)(((int64_t(1) << (n - 5 - 2 * RBf)) + WP_TILES_FWD - 1) / WP_TILES_FWD);
+        P.pfwd.push_back(f);
+      } else if (npf > 0 && w < npf + (int)pa[i].size()) {
+        PairPass a = pa[i][w - npf];
+        a.inst = i;
+        a.block_begin = pab;
+        a.prow = (int32_t)prow;
+        rows[i].push_back(prow);
+        pab += adj_blocks(n);
+        prow += adj_blocks(n);
+        P.padj.push_back(a);
+      } else if (w < nf) {
         WvFwd f = fw[i][w];
         f.inst = i;
         f.block_begin = fb;
@@ -651,8 +769,7 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
         WvAdj a = ad[i][w - nf];
         a.inst = i;
         a.block_begin = ab;
-        const int32_t nb =
-            (int32_t)(((int64_t(1) << (n - 5 - RBa)) + WV_SUBS_PER_BLOCK - 1) / WV_SUBS_PER_BLOCK);
+        const int32_t nb = adj_blocks(n);
         ab += nb;
         a.prow = (int32_t)prow;
         rows[i].push_back(prow);
@@ -664,13 +781,17 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
     wave.adj_count = (int32_t)P.adj.size() - wave.adj_begin;
     wave.fwd_blocks = fb;
     wave.adj_blocks = ab;
+    wave.pfwd_count = (int32_t)P.pfwd.size() - wave.pfwd_begin;
+    wave.padj_count = (int32_t)P.padj.size() - wave.padj_begin;
+    wave.pfwd_blocks = pfb;
+    wave.padj_blocks = pab;
     P.waves.push_back(wave);
   }
   if (prow > INT32_MAX / 2) return QF_ERR_TOO_LARGE;
   // final reduction: per output, the segments of adjoint rows feeding it
   for (int i = 0; i < ninst; ++i) {
-    const int p = P.inst[i].p, n = P.inst[i].n;
-    const int32_t nb = (int32_t)(((int64_t(1) << (n - 5 - RBa)) + WV_SUBS_PER_BLOCK - 1) / WV_SUBS_PER_BLOCK);
+    const int p = P.inst[i].p;
+    const int32_t nb = adj_blocks(P.inst[i].n);
     for (int slot = 0; slot <= 2 * p; ++slot) {
       P.segbeg.push_back((int32_t)P.segs.size());
       P.outidx.push_back(P.inst[i].out_offset + slot);
@@ -683,6 +804,8 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
   P.h.nwaves = nw;
   P.h.nfwd = (int32_t)P.fwd.size();
   P.h.nadj = (int32_t)P.adj.size();
+  P.h.npfwd = (int32_t)P.pfwd.size();
+  P.h.npadj = (int32_t)P.padj.size();
   P.h.nsegs = (int32_t)P.segs.size();
   P.h.nout = (int32_t)P.outidx.size();
   P.h.state_elems = st;
@@ -699,6 +822,8 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
   P.h.off_inst = take(P.inst.size() * sizeof(WvInst));
   P.h.off_fwd = take(P.fwd.size() * sizeof(WvFwd));
   P.h.off_adj = take(P.adj.size() * sizeof(WvAdj));
+  P.h.off_pfwd = take(P.pfwd.size() * sizeof(PairPass));
+  P.h.off_padj = take(P.padj.size() * sizeof(PairPass));
   P.h.off_segbeg = take(P.segbeg.size() * sizeof(int32_t));
   P.h.off_segs = take(P.segs.size() * sizeof(WvSeg));
   P.h.off_outidx = take(P.outidx.size() * sizeof(int32_t));
@@ -710,7 +835,7 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
   // host image: header, waves, then the arrays that are uploaded
   const size_t hbytes = sizeof(WvPlanHeader) + P.waves.size() * sizeof(WvWave) + P.inst.size() * sizeof(WvInst) +
                         P.fwd.size() * sizeof(WvFwd) + P.adj.size() * sizeof(WvAdj) +
-                        P.segbeg.size() * sizeof(int32_t) + P.segs.size() * sizeof(WvSeg) +
+                        (P.pfwd.size() + P.padj.size()) * sizeof(PairPass) + P.segbeg.size() * sizeof(int32_t) + P.segs.size() * sizeof(WvSeg) +
                         P.outidx.size() * sizeof(int32_t);
   if (need_host) *need_host = hbytes;
   if (need_device) *need_device = (size_t)off;
@@ -726,6 +851,8 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
   put(P.inst.data(), P.inst.size() * sizeof(WvInst));
   put(P.fwd.data(), P.fwd.size() * sizeof(WvFwd));
   put(P.adj.data(), P.adj.size() * sizeof(WvAdj));
+  put(P.pfwd.data(), P.pfwd.size() * sizeof(PairPass));
+  put(P.padj.data(), P.padj.size() * sizeof(PairPass));
   put(P.segbeg.data(), P.segbeg.size() * sizeof(int32_t));
   put(P.segs.data(), P.segs.size() * sizeof(WvSeg));
   put(P.outidx.data(), P.outidx.size() * sizeof(int32_t));
@@ -739,6 +866,7 @@ struct PlanView {
   const WvInst* inst;
   const WvFwd* fwd;
   const WvAdj* adj;
+  const PairPass *pfwd, *padj;
   const int32_t* segbeg;
   const WvSeg* segs;
   const int32_t* outidx;
@@ -756,6 +884,10 @@ bool view_plan(const void* host_plan, PlanView& v) {
   h += v.h->nfwd * sizeof(WvFwd);
   v.adj = reinterpret_cast<const WvAdj*>(h);
   h += v.h->nadj * sizeof(WvAdj);
+  v.pfwd = reinterpret_cast<const PairPass*>(h);
+  h += v.h->npfwd * sizeof(PairPass);
+  v.padj = reinterpret_cast<const PairPass*>(h);
+  h += v.h->npadj * sizeof(PairPass);
   v.segbeg = reinterpret_cast<const int32_t*>(h);
   h += (v.h->nout + 1) * sizeof(int32_t);
   v.segs = reinterpret_cast<const WvSeg*>(h);
@@ -778,6 +910,8 @@ int wave_prepare(const void* host_plan, const uint8_t* edges, void* ws, size_t w
   if ((rc = up(h.off_inst, v.inst, h.ninst * sizeof(WvInst)))) return rc;
   if ((rc = up(h.off_fwd, v.fwd, h.nfwd * sizeof(WvFwd)))) return rc;
   if ((rc = up(h.off_adj, v.adj, h.nadj * sizeof(WvAdj)))) return rc;
+  if ((rc = up(h.off_pfwd, v.pfwd, h.npfwd * sizeof(PairPass)))) return rc;
+  if ((rc = up(h.off_padj, v.padj, h.npadj * sizeof(PairPass)))) return rc;
   if ((rc = up(h.off_segbeg, v.segbeg, (h.nout + 1) * sizeof(int32_t)))) return rc;
   if ((rc = up(h.off_segs, v.segs, h.nsegs * sizeof(WvSeg)))) return rc;
   if ((rc = up(h.off_outidx, v.outidx, h.nout * sizeof(int32_t)))) return rc;
@@ -816,6 +950,12 @@ static int wave_run_t(const PlanView& v, char* d, const double* angles, double* 
     rc = check_cuda(cudaFuncSetAttribute(k_wave_adj<LAY, RBA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(smem_max + wv_ring_bytes<LAY, RBA>(2))));
     if (rc) return rc;
+    rc = check_cuda(cudaFuncSetAttribute(k_wave_pair_fwd<LAY, RBF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(smem_max + 2 * PairShape<LAY, RBF>::VEC)));
+    if (rc) return rc;
+    rc = check_cuda(cudaFuncSetAttribute(k_wave_pair_adj<LAY, RBA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(smem_max + 3 * PairShape<LAY, RBA>::VEC)));
+    if (rc) return rc;
     attr[dev].store(true);
   }
   k_wave_coefs<LAY><<<h.ninst, 128, 0, stream>>>(dinst, h.ninst, angles, const_cast<Coef*>(dtab), skip);
@@ -823,11 +963,25 @@ static int wave_run_t(const PlanView& v, char* d, const double* angles, double* 
   if (rc) return rc;
   const WvFwd* dfwd = reinterpret_cast<const WvFwd*>(d + h.off_fwd);
   const WvAdj* dadj = reinterpret_cast<const WvAdj*>(d + h.off_adj);
+  const PairPass* dpf = reinterpret_cast<const PairPass*>(d + h.off_pfwd);
+  const PairPass* dpa = reinterpret_cast<const PairPass*>(d + h.off_padj);
   for (int w = 0; w < h.nwaves; ++w) {
     const WvWave& W = v.waves[w];
     if (W.fwd_count > 0) {
       k_wave_fwd<LAY, RBF><<<W.fwd_blocks, 256, smem_f, stream>>>(
           dfwd + W.fwd_begin, W.fwd_count, dinst, dstates, dcuts, dtab, (int)cutb, skip);
+      if ((rc = check_cuda(cudaGetLastError()))) return rc;
+    }
+    if (W.pfwd_count > 0) {
+      k_wave_pair_fwd<LAY, RBF><<<W.pfwd_blocks, PairShape<LAY, RBF>::NT, cutb + 2 * PairShape<LAY, RBF>::VEC,
+                                  stream>>>(dpf + W.pfwd_begin, W.pfwd_count, dinst, dstates, dcuts, dtab, (int)cutb,
+                                            skip);
+      if ((rc = check_cuda(cudaGetLastError()))) return rc;
+    }
+    if (W.padj_count > 0) {
+      k_wave_pair_adj<LAY, RBA><<<W.padj_blocks, PairShape<LAY, RBA>::NT, cutb + 3 * PairShape<LAY, RBA>::VEC,
+                                  stream>>>(dpa + W.padj_begin, W.padj_count, dinst, dstates, dcuts, dtab, dpart,
+                                            (int)cutb, skip);
       if ((rc = check_cuda(cudaGetLastError()))) return rc;
     }
     if (W.adj_count > 0) {
