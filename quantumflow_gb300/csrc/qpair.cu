@@ -6,8 +6,8 @@
 // warp-tile passes these replace from 13 qubits on: the same operations in
 // the same order, half of the passes over the state.
 // Bound: HBM (adjoint passes, 106 us at n = 24 of 80 at the copy rate); the
-// forward passes, 69 us of 40, FP32 issue and shuffles at the layer
-// boundaries.  n = 24, p = 6: 4956 -> 3074 us a gradient evaluation
+// forward passes, 66 us of 40, FP32 issue and shuffles at the layer
+// boundaries.  n = 24, p = 6: 4956 -> 3050 us a gradient evaluation
 // (forward 25 passes -> 13, adjoint 37 -> 19).
 #include <algorithm>
 #include <atomic>
@@ -47,10 +47,10 @@ QF_D unsigned char* qp_table(const QPairParams& P, unsigned char* smem) {
   return smem + ((P.ncut * sizeof(Coef) + 127) & ~size_t(127));
 }
 
-__global__ void __launch_bounds__(PairShape<C64, QP_RBF>::NT, 1) k_qpair_fwd(const __grid_constant__ QPairParams P) {
+__global__ void __launch_bounds__(PairShape<C64, QP_RBF>::NT, 2) k_qpair_fwd(const __grid_constant__ QPairParams P) {
   extern __shared__ __align__(128) unsigned char qp_smem[];
   unsigned char* buf = qp_table(P, qp_smem);
-  pair_forward<C64, QP_RBF>(P.F, P.psi, P.cuts, reinterpret_cast<const Coef*>(qp_smem), P.ncut,
+  pair_forward<C64, QP_RBF, false>(P.F, P.psi, P.cuts, reinterpret_cast<const Coef*>(qp_smem), P.ncut,
                             make_float2(P.amp0.f[0], P.amp0.f[2]), P.ac, P.as, P.bc, P.bs, blockIdx.x, gridDim.x,
                             1u << (P.n - 5 - 2 * QP_RBF), buf);
 }
@@ -94,7 +94,7 @@ int qp_attr() {
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || attr[dev].load()) return QF_OK;
   int rc = check_cuda(cudaFuncSetAttribute(k_qpair_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)qp_smem<QP_RBF>(1, QP_MAX_COEF)));
+                                           (int)qp_smem<QP_RBF>(0, QP_MAX_COEF)));
   if (rc) return rc;
   rc = check_cuda(cudaFuncSetAttribute(k_qpair_adj, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)qp_smem<QP_RBA>(2, QP_MAX_COEF)));
@@ -127,7 +127,7 @@ int qpair_state(void* psi, int n, const uint16_t* cuts, int nedges, int p, const
     c = make_coef(cplx(std::cos(0.5 * beta[l]), 0.0), C64);
     s = make_coef(cplx(-std::sin(0.5 * beta[l]), 0.0), C64);
   };
-  const int grid = qp_grid(n, QP_RBF, 1);
+  const int grid = qp_grid(n, QP_RBF, 2);
   for (const PairPass& F : pair_fwd_passes(n, p, QP_RBF)) {
     P.F = F;
     if (F.hasA) rx(F.layerA, P.ac, P.as);
@@ -136,7 +136,7 @@ int qpair_state(void* psi, int n, const uint16_t* cuts, int nedges, int p, const
       for (int cv = 0; cv <= nedges; ++cv)
         P.coef[cv] = make_coef(std::polar(1.0, gamma[F.layerB] * (0.5 * nedges - cv)), C64);
     }
-    k_qpair_fwd<<<grid, PairShape<C64, QP_RBF>::NT, qp_smem<QP_RBF>(1, P.ncut), stream>>>(P);
+    k_qpair_fwd<<<grid, PairShape<C64, QP_RBF>::NT, qp_smem<QP_RBF>(0, P.ncut), stream>>>(P);
     if ((rc = check_cuda(cudaGetLastError()))) return rc;
   }
   return QF_OK;

@@ -279,9 +279,14 @@ QF_D void pair_mix(const Coef& c, const Coef& s, bool lanes, int nact, E (&a)[1 
   if constexpr (F32) acc.add(part, 0.f);
 }
 
+// PREF: the next tile's amplitudes are fetched into thread-private slots while
+// a tile is worked on; else two CTAs per SM overlap each other's loads, which
+// the tile of 2^13 complex64 amplitudes leaves room for only without the
+// slots (32 graphs of 20 qubits, p = 6: 3474 us an evaluation with them, 2961
+// without; float-float, whose tiles are smaller, the other way round).
 // Forward pass over the tiles first, first + stride, ... < ntiles.  ac .. bs:
 // RX of mixer A and B; tab: the cost layer's phases (shared memory).
-template <int LAY, int RB>
+template <int LAY, int RB, bool PREF>
 QF_D void pair_forward(const PairPass& F, typename Types<LAY>::E* psi, const uint16_t* cuts, const Coef* tab, int ncut,
                        typename Types<LAY>::E amp0, const Coef& ac, const Coef& as, const Coef& bc, const Coef& bs,
                        uint32_t first, uint32_t stride, uint32_t ntiles, unsigned char* smem) {
@@ -294,6 +299,7 @@ QF_D void pair_forward(const PairPass& F, typename Types<LAY>::E* psi, const uin
   E* next = reinterpret_cast<E*>(smem + S::VEC) + threadIdx.x;  // this thread's slots: register * NT
   const bool xfirst = F.pair && F.hasA;  // arrangement at load: X in registers, else Y
   auto fetch = [&](uint32_t tile) {
+    if constexpr (!PREF) return;
     if (tile < ntiles && !F.init) {
       const uint32_t b = G.base(tile, lane) | (xfirst ? G.wy : G.wx);
 #pragma unroll
@@ -306,18 +312,26 @@ QF_D void pair_forward(const PairPass& F, typename Types<LAY>::E* psi, const uin
     const uint32_t b = G.base(tile, lane);
     const uint32_t by = b | G.wx;  // Y in registers
     int cv[R];
-    if (F.cost) {
+    if constexpr (PREF) {
+      if (F.cost) {  // on their way while the tile is awaited
 #pragma unroll
-      for (int r = 0; r < R; ++r) cv[r] = cuts[by | G.offy(r)];
+        for (int r = 0; r < R; ++r) cv[r] = cuts[by | G.offy(r)];
+      }
+      cp_async_wait<0>();
     }
-    cp_async_wait<0>();
     E a[R];
     if (F.init) {
 #pragma unroll
       for (int r = 0; r < R; ++r) a[r] = amp0;
-    } else {
+    } else if constexpr (PREF) {
 #pragma unroll
       for (int r = 0; r < R; ++r) a[r] = next[r * S::NT];
+    } else if (xfirst) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[r] = psi[b | G.wy | G.offx(r)];
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[r] = psi[by | G.offy(r)];
     }
     bool xnow = xfirst;
     if (F.hasA) {
@@ -333,7 +347,7 @@ QF_D void pair_forward(const PairPass& F, typename Types<LAY>::E* psi, const uin
     }
     if (F.cost) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) a[r] = cmul_v(tab[min(cv[r], ncut - 1)], a[r]);
+      for (int r = 0; r < R; ++r) a[r] = cmul_v(tab[min(PREF ? cv[r] : (int)cuts[by | G.offy(r)], ncut - 1)], a[r]);
     }
     if (F.hasB) {
       pair_rx<RB>(bc, bs, true, F.ny, a);

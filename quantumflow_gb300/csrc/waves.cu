@@ -8,7 +8,7 @@
 // one pass.  Instances of at least a two-group tile (complex64 13 qubits,
 // float-float 11) take two register groups a pass (qpair.cuh: the same
 // operations in the same order, a third to a half of the passes).  200 graphs
-// of 8 to 18 qubits, complex64: 2295 -> 1545 us of kernels an evaluation.  Wave w launches the w-th pass of every instance that has
+// of 8 to 18 qubits, complex64: 2295 -> 1461 us of kernels an evaluation.  Wave w launches the w-th pass of every instance that has
 // one -- forward items in one launch, adjoint items in another -- so one
 // launch covers all instances and the launch count is the longest
 // instance's pass count, whatever the batch size.  Every launch reads its
@@ -477,8 +477,12 @@ QF_D bool wp_begin(const PairPass* items, int nitems, const WvInst* inst, const 
   return true;
 }
 
+// (Blocks per SM for the register allocation: complex64 2 and 3, against 1 and
+// 2 that the compiler's own choice allows, 200 graphs 1545 -> 1450 us.  In
+// float-float any minimum costs more than it gives: 4994 us without, 5460 with
+// 3 and 5.)
 template <int LAY, int RB>
-__global__ void __launch_bounds__(PairShape<LAY, RB>::NT) k_wave_pair_fwd(const PairPass* items, int nitems,
+__global__ void __launch_bounds__(PairShape<LAY, RB>::NT, LAY == C64 ? 2 : 0) k_wave_pair_fwd(const PairPass* items, int nitems,
                                                                           const WvInst* inst, void* states,
                                                                           const uint16_t* cuts, const Coef* tab,
                                                                           int cutb, const int32_t* skip) {
@@ -493,12 +497,12 @@ __global__ void __launch_bounds__(PairShape<LAY, RB>::NT) k_wave_pair_fwd(const 
   const E amp0 = coef_e(wv_coef<LAY>(1.0 / sqrt((double)(int64_t(1) << I.n)), 0.0), tag);
   const uint32_t first = (blockIdx.x - F.block_begin) * WP_TILES_FWD, all = 1u << (I.n - 5 - 2 * RB);
   const Coef ac = t[3 * F.layerA], as = t[3 * F.layerA + 1], bc = t[3 * F.layerB], bs = t[3 * F.layerB + 1];
-  pair_forward<LAY, RB>(F, reinterpret_cast<E*>(states) + I.psi, cuts + I.cuts, scut, I.nedges + 1, amp0, ac, as, bc,
+  pair_forward<LAY, RB, LAY != C64>(F, reinterpret_cast<E*>(states) + I.psi, cuts + I.cuts, scut, I.nedges + 1, amp0, ac, as, bc,
                         bs, first, 1u, min(first + WP_TILES_FWD, all), smem_raw + cutb);
 }
 
 template <int LAY, int RB>
-__global__ void __launch_bounds__(PairShape<LAY, RB>::NT) k_wave_pair_adj(const PairPass* items, int nitems,
+__global__ void __launch_bounds__(PairShape<LAY, RB>::NT, LAY == C64 ? 3 : 0) k_wave_pair_adj(const PairPass* items, int nitems,
                                                                           const WvInst* inst, void* states,
                                                                           const uint16_t* cuts, const Coef* tab,
                                                                           double* partials, int cutb,
@@ -973,7 +977,7 @@ static int wave_run_t(const PlanView& v, char* d, const double* angles, double* 
       if ((rc = check_cuda(cudaGetLastError()))) return rc;
     }
     if (W.pfwd_count > 0) {
-      k_wave_pair_fwd<LAY, RBF><<<W.pfwd_blocks, PairShape<LAY, RBF>::NT, cutb + 2 * PairShape<LAY, RBF>::VEC,
+      k_wave_pair_fwd<LAY, RBF><<<W.pfwd_blocks, PairShape<LAY, RBF>::NT, cutb + (LAY == C64 ? 1 : 2) * PairShape<LAY, RBF>::VEC,
                                   stream>>>(dpf + W.pfwd_begin, W.pfwd_count, dinst, dstates, dcuts, dtab, (int)cutb,
                                             skip);
       if ((rc = check_cuda(cudaGetLastError()))) return rc;
