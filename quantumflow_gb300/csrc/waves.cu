@@ -558,7 +558,11 @@ __global__ void k_wave_reduce(const int32_t* seg_begin, const WvSeg* segs, int n
 // ------------------------------------------------------------ host plan ----
 struct WvPlanHeader {
   int32_t magic, layout, rbf, rba;
-  int32_t ninst, nwaves, nfwd, nadj, npfwd, npadj, nsegs, nout;
+  // the schedule in passes of one register group: per instance
+  // 1 + p (m - 1) a sweep (a two-group pass stands for the ones it covers)
+  int32_t ninst, nwaves, nfwd, nadj, nsegs, nout;
+  // the passes that run: waves (launch rounds), one-group and two-group items
+  int32_t rounds, ifwd, iadj, ipfwd, ipadj, pad;
   int64_t state_elems, cut_elems, tab_coefs, prows;
   // device byte offsets inside the workspace
   int64_t off_inst, off_fwd, off_adj, off_pfwd, off_padj, off_segbeg, off_segs, off_outidx, off_tab, off_part, off_cuts, off_states;
@@ -570,7 +574,7 @@ struct WvWave {
   int32_t pfwd_begin, pfwd_count, pfwd_blocks;  // two register groups a pass
   int32_t padj_begin, padj_count, padj_blocks;
 };
-constexpr int32_t WV_MAGIC = 0x51465757;  // the version of this layout
+constexpr int32_t WV_MAGIC = 0x51465758;  // the version of this layout
 
 static int wv_rb_fwd(int layout) { return layout == C64 ? 4 : 3; }
 static int wv_rb_adj(int layout) { return layout == C64 ? 3 : 2; }
@@ -702,7 +706,7 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
     return (int32_t)(((int64_t(1) << (n - 5 - (pairs(n) ? 2 : 1) * RBa)) + per - 1) / per);
   };
   int64_t st = 0, ct = 0, tb = 0;
-  int nw = 0;
+  int nw = 0, nfwd1 = 0, nadj1 = 0, nw1 = 0;
   for (int i = 0; i < ninst; ++i) {
     const qf_batch_instance& q = hinst[i];
     if (q.n < wave_min_qubits(layout) || q.n > QF_MAX_QUBITS || q.p < 1 || q.p > 64 || q.nedges < 0 ||
@@ -724,14 +728,19 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
     w.tab = tb;
     tb += wv_tab_size(q.p, q.nedges);
     P.inst.push_back(w);
+    wv_fwd_passes(q.n, q.p, RBf, fw[i]);
+    wv_adj_passes(q.n, q.p, RBa, ad[i], sl[i]);
+    nfwd1 += (int)fw[i].size();
+    nadj1 += (int)ad[i].size();
+    nw1 = std::max(nw1, (int)(fw[i].size() + ad[i].size()));
     if (pairs(q.n)) {
+      fw[i].clear();
+      ad[i].clear();
+      sl[i].clear();
       pf[i] = pair_fwd_passes(q.n, q.p, RBf);
       pa[i] = pair_adj_passes(q.n, q.p, RBa);
       for (const PairPass& a : pa[i])
         sl[i].push_back({q.p + a.layerA, a.cost ? a.layerA : -1, a.init ? 2 * q.p : -1, a.hasB ? q.p + a.layerB : -1});
-    } else {
-      wv_fwd_passes(q.n, q.p, RBf, fw[i]);
-      wv_adj_passes(q.n, q.p, RBa, ad[i], sl[i]);
     }
     nw = std::max(nw, (int)(fw[i].size() + ad[i].size() + pf[i].size() + pa[i].size()));
   }
@@ -805,11 +814,14 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
     }
   }
   P.segbeg.push_back((int32_t)P.segs.size());
-  P.h.nwaves = nw;
-  P.h.nfwd = (int32_t)P.fwd.size();
-  P.h.nadj = (int32_t)P.adj.size();
-  P.h.npfwd = (int32_t)P.pfwd.size();
-  P.h.npadj = (int32_t)P.padj.size();
+  P.h.nwaves = nw1;
+  P.h.nfwd = nfwd1;
+  P.h.nadj = nadj1;
+  P.h.rounds = nw;
+  P.h.ifwd = (int32_t)P.fwd.size();
+  P.h.iadj = (int32_t)P.adj.size();
+  P.h.ipfwd = (int32_t)P.pfwd.size();
+  P.h.ipadj = (int32_t)P.padj.size();
   P.h.nsegs = (int32_t)P.segs.size();
   P.h.nout = (int32_t)P.outidx.size();
   P.h.state_elems = st;
@@ -881,17 +893,17 @@ bool view_plan(const void* host_plan, PlanView& v) {
   if (v.h->magic != WV_MAGIC) return false;
   h += sizeof(WvPlanHeader);
   v.waves = reinterpret_cast<const WvWave*>(h);
-  h += v.h->nwaves * sizeof(WvWave);
+  h += v.h->rounds * sizeof(WvWave);
   v.inst = reinterpret_cast<const WvInst*>(h);
   h += v.h->ninst * sizeof(WvInst);
   v.fwd = reinterpret_cast<const WvFwd*>(h);
-  h += v.h->nfwd * sizeof(WvFwd);
+  h += v.h->ifwd * sizeof(WvFwd);
   v.adj = reinterpret_cast<const WvAdj*>(h);
-  h += v.h->nadj * sizeof(WvAdj);
+  h += v.h->iadj * sizeof(WvAdj);
   v.pfwd = reinterpret_cast<const PairPass*>(h);
-  h += v.h->npfwd * sizeof(PairPass);
+  h += v.h->ipfwd * sizeof(PairPass);
   v.padj = reinterpret_cast<const PairPass*>(h);
-  h += v.h->npadj * sizeof(PairPass);
+  h += v.h->ipadj * sizeof(PairPass);
   v.segbeg = reinterpret_cast<const int32_t*>(h);
   h += (v.h->nout + 1) * sizeof(int32_t);
   v.segs = reinterpret_cast<const WvSeg*>(h);
@@ -912,10 +924,10 @@ int wave_prepare(const void* host_plan, const uint8_t* edges, void* ws, size_t w
   };
   int rc;
   if ((rc = up(h.off_inst, v.inst, h.ninst * sizeof(WvInst)))) return rc;
-  if ((rc = up(h.off_fwd, v.fwd, h.nfwd * sizeof(WvFwd)))) return rc;
-  if ((rc = up(h.off_adj, v.adj, h.nadj * sizeof(WvAdj)))) return rc;
-  if ((rc = up(h.off_pfwd, v.pfwd, h.npfwd * sizeof(PairPass)))) return rc;
-  if ((rc = up(h.off_padj, v.padj, h.npadj * sizeof(PairPass)))) return rc;
+  if ((rc = up(h.off_fwd, v.fwd, h.ifwd * sizeof(WvFwd)))) return rc;
+  if ((rc = up(h.off_adj, v.adj, h.iadj * sizeof(WvAdj)))) return rc;
+  if ((rc = up(h.off_pfwd, v.pfwd, h.ipfwd * sizeof(PairPass)))) return rc;
+  if ((rc = up(h.off_padj, v.padj, h.ipadj * sizeof(PairPass)))) return rc;
   if ((rc = up(h.off_segbeg, v.segbeg, (h.nout + 1) * sizeof(int32_t)))) return rc;
   if ((rc = up(h.off_segs, v.segs, h.nsegs * sizeof(WvSeg)))) return rc;
   if ((rc = up(h.off_outidx, v.outidx, h.nout * sizeof(int32_t)))) return rc;
@@ -969,7 +981,7 @@ static int wave_run_t(const PlanView& v, char* d, const double* angles, double* 
   const WvAdj* dadj = reinterpret_cast<const WvAdj*>(d + h.off_adj);
   const PairPass* dpf = reinterpret_cast<const PairPass*>(d + h.off_pfwd);
   const PairPass* dpa = reinterpret_cast<const PairPass*>(d + h.off_padj);
-  for (int w = 0; w < h.nwaves; ++w) {
+  for (int w = 0; w < h.rounds; ++w) {
     const WvWave& W = v.waves[w];
     if (W.fwd_count > 0) {
       k_wave_fwd<LAY, RBF><<<W.fwd_blocks, 256, smem_f, stream>>>(
