@@ -134,7 +134,8 @@ int qf_set_gate_merging(int on);
  * or qubit-exchange pass,
  * 1 direct single-gate sweep, 2 fused warp-tile or shared-memory pass,
  * 3 group pass, 4 shape pass, 5 one gate in native FP64 inside a
- * QF_LAYOUT_FX circuit, 6 tensor-core complex128 pass).  *nblocks gets the pass count; at most max_blocks
+ * QF_LAYOUT_FX circuit, 6 tensor-core complex128 pass, 7 complex64 pass on
+ * wide tiles).  *nblocks gets the pass count; at most max_blocks
  * rows are written. */
 int qf_plan_circuit(int n, int layout, int nops, const int* op_k, const int* op_axes, const double* op_mats,
                     int fusion_k, int32_t* stats, int max_blocks, int* nblocks);

@@ -6,6 +6,7 @@
 // and write the ket axes back in place -- applied in list order as
 // quantumflow/circuits.py:87-99 Circuit.run does.  Nothing here is a
 // translation of that einsum: the state is swept once per fused block.
+#include "cwide.cuh"
 #include "engine.cuh"
 #include "regops.cuh"
 
@@ -1992,7 +1993,48 @@ struct PlanBlock {
   uint64_t hmask = 0;
   int ncoef = 0;
   bool elem_only = true;
+  std::vector<std::vector<int>> stages;  // complex64: a pass on wide tiles (cwide.cu)
 };
+
+// Runs of complex64 blocks of 2x2 and 4x4 gates and signs become passes on
+// wide tiles where that takes at most five for six of them (n = 26: a wide
+// pass of two gates about 1.1 shape passes, of six 2.2).
+static void widen_blocks(std::vector<PlanBlock>& blocks, const std::vector<HostOp>& ops, int n) {
+  std::vector<PlanBlock> out;
+  out.reserve(blocks.size());
+  for (size_t i = 0; i < blocks.size();) {
+    size_t end = i;
+    std::vector<int> idx;
+    for (; end < blocks.size(); ++end) {
+      bool ok = true;
+      for (int k : blocks[end].idx) ok = ok && cwide_op(ops[k]);
+      if (!ok) break;
+      idx.insert(idx.end(), blocks[end].idx.begin(), blocks[end].idx.end());
+    }
+    if (end - i >= 2) {
+      std::vector<CWidePass> passes = cwide_plan(ops, idx, n);
+      if (passes.size() * 6 <= (end - i) * 5) {
+        for (CWidePass& p : passes) {
+          PlanBlock b;
+          b.elem_only = false;
+          b.stages = std::move(p.stages);
+          for (const auto& st : b.stages)
+            for (int k : st) {
+              b.idx.push_back(k);
+              if (!is_elementwise(ops[k].type))
+                for (int j = 0; j < ops[k].k; ++j) b.hmask |= uint64_t(1) << ops[k].gb[j];
+            }
+          out.push_back(std::move(b));
+        }
+        i = end;
+        continue;
+      }
+    }
+    do out.push_back(std::move(blocks[i++]));
+    while (i < end);
+  }
+  blocks.swap(out);
+}
 
 // Float-float fused passes of dense gates and sign ops are cut where their
 // next dense gate would leave the shape table (group.cu), so that each
@@ -2055,6 +2097,7 @@ static void split_for_shapes(std::vector<PlanBlock>& blocks, const std::vector<H
 // Gate merging, then greedy blocking into passes (see above); host only.
 static std::vector<PlanBlock> plan_blocks(std::vector<HostOp>& ops, int n, int layout, int& fusion_k) {
   const int Lmin = 5;  // bits 0..4 are the lane bits of every fused kernel
+  const bool standard = fusion_k <= 0;
   if (fusion_k <= 0) fusion_k = g_default_fusion[layout];
   if (fusion_k > 8) fusion_k = 8;
   if (fusion_k > 1 && g_merge_gates) merge_ops(ops, n);
@@ -2088,6 +2131,8 @@ static std::vector<PlanBlock> plan_blocks(std::vector<HostOp>& ops, int n, int l
   // N=28 against 0.67 ms per two-gate shape pass
   if (layout == C64 && group_pass_enabled() && shape_max_bits(C64) > 0)
     split_for_shapes(blocks, ops, shape_max_bits(C64), 2);
+  if (layout == C64 && standard && group_pass_enabled() && shape_max_bits(C64) > 0 && cwide_fits(n))
+    widen_blocks(blocks, ops, n);
   return blocks;
 }
 
@@ -2115,6 +2160,10 @@ int plan_stats(int n, int layout, std::vector<HostOp>& ops, int fusion_k, int32_
       else st[5]++;
     }
     st[6] = __builtin_popcountll(B.hmask & ~uint64_t(31));
+    if (!B.stages.empty()) {
+      st[7] = 7;
+      continue;
+    }
     const HostOp& first = ops[B.idx[0]];
     st[7] = B.elem_only ? 0
             : (B.idx.size() == 1 && (first.type == OP_DENSE1 || first.type == OP_MONO || first.type == OP_DENSE2))
@@ -2150,7 +2199,10 @@ int run_ops(const void* in, void* out, int n, int layout, std::vector<HostOp>& o
   for (const PlanBlock& b : blocks) {
     int rc;
     const HostOp& first = ops[b.idx[0]];
-    if (b.elem_only) {
+    if (!b.stages.empty()) {
+      LaunchTimer timer(QF_KERNEL_SHAPE, stream);
+      rc = cwide_run(src, out, n, ops, CWidePass{b.stages}, stream);
+    } else if (b.elem_only) {
       LaunchTimer timer(QF_KERNEL_ELEMENTWISE, stream);
       rc = launch_elem(src, out, n, layout, ops, b.idx, stream);
     } else if (b.idx.size() == 1 &&
