@@ -147,8 +147,8 @@ class Circuit(Operation):
         from .densities import evolve_gates
         if rho is None:
             rho = zero_state(self.qubits).asdensity()
-        # channels join the launch where the planner keeps them apart from
-        # the unitary gates (fixed point) or a merged pass costs the same
+        # channels join the launch where the planner takes them into a gate
+        # pass or runs them in FP64 (fixed point) or a merged pass costs the same
         join = rho.dtype == "complex64" or config.C128_ARITHMETIC == "fx"
         pending = []
         for elem in self.gates():

@@ -339,10 +339,11 @@ struct TxParams {
   const void* in;
   void* out;
   int* err;
-  int32_t n, nin, nout, pad;
+  int32_t n, nin, nout;
+  int32_t shift;                    // U is stored scaled by 2^-shift (0 for a unitary)
   int32_t sbits[4];                 // window bits, ascending
   int64_t off[16];                  // global offset of window index c
-  int64_t g[16][16][2];             // U as round(entry * 2^62): [out c][in c][re, im]
+  int64_t g[16][16][2];             // U as round(entry * 2^(62 - shift)): [out c][in c][re, im]
   uint64_t in_mout[TX_MAX_SIGNS];   // input-side sign ops: their bits outside the window
   uint64_t out_mout[TX_MAX_SIGNS];  // output-side sign ops
   uint16_t in_rmask[TX_MAX_SIGNS];  // window indices c that carry all of the op's window bits

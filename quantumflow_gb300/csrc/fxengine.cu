@@ -666,6 +666,46 @@ bool tx_wide(const HostOp& op) {
   return false;
 }
 
+// The squared norm bound of an op that a tensor-core window takes although
+// it is not unitary (the superoperators of noise channels, mostly), or 0
+// when it takes none.  Three conditions:
+//  * every diagonal entry exceeds the rest of its row by at least 1/2, so
+//    that the inverse has row sums of at most 2: an output that is small
+//    beside its row's inputs is then no more a difference of large ones
+//    than behind a gate, and the row's shared exponent serves it as well
+//    (a strong damping or a projection keeps the native FP64 kernels);
+//  * |M|_1 |M|_inf, which bounds the square of the 2-norm, is at most 4;
+//  * no entry but 0 is below 2^-12, of which the window's 2^-62 grid would
+//    keep fewer than 50 bits.
+double tx_channel(const HostOp& op) {
+  const int D = 1 << op.k;
+  if (op.type == OP_DIAG && op.k <= 3) {
+    double big = 0.0;
+    for (int r = 0; r < D; ++r) {
+      const double a = std::abs(op.diag[r]);
+      if (!(a >= 0.5)) return 0.0;
+      big = std::max(big, a);
+    }
+    return big <= 2.0 ? big * big : 0.0;
+  }
+  if (op.type != OP_DENSE1 && op.type != OP_DENSE2 && !(op.type == OP_DENSEK && op.k <= 4)) return 0.0;
+  double row = 0.0, col[16] = {0.0};
+  for (int r = 0; r < D; ++r) {
+    double off = 0.0;
+    for (int c = 0; c < D; ++c) {
+      const double a = std::abs(op.m[r * D + c]);
+      if (a > 0.0 && a < 0x1p-12) return 0.0;
+      col[c] += a;
+      if (c != r) off += a;
+    }
+    const double d = std::abs(op.m[r * D + r]);
+    if (!(d >= off + 0.5)) return 0.0;
+    row = std::max(row, d + off);
+  }
+  const double bound = row * *std::max_element(col, col + D);
+  return bound <= 4.0 ? bound : 0.0;
+}
+
 constexpr int FX_G_MAX = 4;
 
 // Greedy passes: element-wise ops join the current pass; a dense op joins
@@ -711,7 +751,11 @@ bool is_swap(const HostOp& op) {
 // tensor-core passes) the group kernel's limits on element-wise ops do not
 // apply, 3- and 4-qubit unitary gates become blocks of their own, and so do
 // runs of at least three disjoint SWAPs: one exchange pass (n = 23: 70 us)
-// against one tensor-core pass (69 us) per two of them.
+// against one tensor-core pass (69 us) per two of them.  Where the list has
+// channels a pass can take (tx_channel), a dense gate and its image on the
+// bits a constant distance away (the ket and bra sides of a density) stay in
+// one window, which then takes the channels on those qubits: two layers with
+// a channel per qubit, 11 qubits: 12 passes instead of 32.
 std::vector<FxBlock> fx_blocks(const std::vector<HostOp>& ops, const std::vector<int>& list, int fusion_k,
                                bool tensor) {
   const int gmax = std::min(fusion_k, FX_G_MAX);
@@ -722,6 +766,15 @@ std::vector<FxBlock> fx_blocks(const std::vector<HostOp>& ops, const std::vector
     if (!cur.idx.empty()) blocks.push_back(cur);
     cur = FxBlock();
   };
+  bool channels = false;
+  if (tensor && fuse)
+    for (int i : list) channels = channels || (fx_kind(ops[i]) == FXK_NATIVE && tx_channel(ops[i]) > 0.0);
+  auto image = [&](const HostOp& a, const HostOp& b) {
+    if (fx_kind(b) != FXK_DENSE || a.k != b.k || a.k > 2) return false;
+    const int d = b.gb[0] - a.gb[0];
+    return d != 0 && (a.k == 1 || b.gb[1] - a.gb[1] == d);
+  };
+  bool second = false;  // the op is the image of the one before it
   for (size_t li = 0; li < list.size(); ++li) {
     const int i = list[li];
     const HostOp& op = ops[i];
@@ -763,7 +816,17 @@ std::vector<FxBlock> fx_blocks(const std::vector<HostOp>& ops, const std::vector
     if (kind == FXK_DENSE)
       for (int j = 0; j < op.k; ++j)
         if (std::find(cur.order, cur.order + cur.G, op.gb[j]) == cur.order + cur.G) add[nadd++] = op.gb[j];
-    const bool fits = cur.G + nadd <= gmax && (tensor || ((int)cur.idx.size() < FXG_MAX_OPS / 3 &&
+    const bool first = channels && !second && kind == FXK_DENSE && 2 * op.k <= gmax && li + 1 < list.size() &&
+                       image(op, ops[list[li + 1]]);
+    int both = cur.G + nadd;
+    if (first) {
+      const HostOp& im = ops[list[li + 1]];
+      for (int j = 0; j < im.k; ++j)
+        both += std::find(cur.order, cur.order + cur.G, im.gb[j]) == cur.order + cur.G &&
+                std::find(add, add + nadd, im.gb[j]) == add + nadd;
+    }
+    second = first;
+    const bool fits = both <= gmax && (tensor || ((int)cur.idx.size() < FXG_MAX_OPS / 3 &&
                                                           cur.ncoef + need <= FXG_MAX_COEF));
     if (!cur.idx.empty() && (!fuse || !fits)) close();
     if (kind == FXK_DENSE) {
@@ -1155,10 +1218,10 @@ inline int64_t round62(i128 v) { return static_cast<int64_t>((v + (i128(1) << 61
 struct TxUnitary {
   int64_t re[16][16], im[16][16];
   uint32_t used = 0;  // window bits of the gates so far
-  void identity() {
+  void identity(int shift) {
     std::memset(re, 0, sizeof(re));
     std::memset(im, 0, sizeof(im));
-    for (int c = 0; c < 16; ++c) re[c][c] = int64_t(1) << 62;
+    for (int c = 0; c < 16; ++c) re[c][c] = int64_t(1) << (62 - shift);
     used = 0;
   }
   // f(r, c) for the entries that can be nonzero
@@ -1237,6 +1300,9 @@ struct TxUnitary {
 // touches its window bits, else to the outputs when no later one does.
 // With `matrix` false only the structure is checked (the planner's test);
 // with it, U is multiplied up from the gates in block order (TxUnitary).
+// Ops that tx_channel admits make U's norm at most 2 (their bounds'
+// product): it is then held halved, so that its rows keep a unitary's
+// bounds, and the outputs' exponent is one higher.
 int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams& P, bool matrix = true) {
   if (B.native || B.G < 1 || B.G > 4 || n < 11) return QF_ERR_NOT_SUPPORTED;
   auto dense_op = [](const HostOp& op) {
@@ -1262,8 +1328,17 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
       if ((c >> j) & 1) o |= int64_t(1) << wb[j];
     P.off[c] = o;
   }
+  double norm2 = 1.0;
+  for (int i : B.idx) {
+    if (fx_kind(ops[i]) != FXK_NATIVE || tx_wide(ops[i])) continue;
+    const double b = tx_channel(ops[i]);
+    if (b == 0.0) return QF_ERR_NOT_SUPPORTED;
+    norm2 *= std::max(b, 1.0);
+  }
+  if (norm2 > 4.0) return QF_ERR_NOT_SUPPORTED;
+  P.shift = norm2 > 1.0 + FX_UNIT_TOL ? 1 : 0;
   static thread_local TxUnitary U;
-  if (matrix) U.identity();
+  if (matrix) U.identity(P.shift);
   // window bits each dense op of the block touches, for the sign placement
   std::vector<int> dense_pos;
   std::vector<uint32_t> dense_bits;
@@ -1278,7 +1353,6 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
   }
   for (int k = 0; k < (int)B.idx.size(); ++k) {
     const HostOp& op = ops[B.idx[k]];
-    if (fx_kind(op) == FXK_NATIVE && !tx_wide(op)) return QF_ERR_NOT_SUPPORTED;
     if (dense_op(op)) {
       int jp[4];
       for (int j = 0; j < op.k; ++j) {
@@ -1668,6 +1742,43 @@ void plan_tensor_block(const std::vector<HostOp>& ops, int n, const FxBlock& who
   }
 }
 
+// A native op that tx_channel admits joins the latest tensor-core pass on
+// its bits when that pass's window has them all and the passes between do
+// not touch them: the pass costs the same, and the sweep of its own goes
+// (n = 22: 36 us for a depolarizing channel, 23 for a dephasing one, beside
+// 31 for the pass).  Two layers with a channel per qubit, 11 qubits: 1065 ->
+// 665 us a call, 3 layers on 12 qubits 5.2 -> 2.3 ms; error against 80-bit
+// arithmetic 4.4e-16 -> 3.7e-16.  Never a pass of channels alone: it would
+// hold their rows to a shared exponent that no gate asks for, and gain little
+// (31 us against two sweeps).
+void absorb_channels(const std::vector<HostOp>& ops, int n, std::vector<FxBlock>& blocks) {
+  static thread_local TxParams tp;
+  size_t kept = 0;
+  for (size_t b = 0; b < blocks.size(); ++b) {
+    bool gone = false;
+    if (blocks[b].native && tx_channel(ops[blocks[b].idx[0]]) > 0.0) {
+      const int i = blocks[b].idx[0];
+      const uint64_t bits = op_bits(ops[i]);
+      for (size_t t = kept; t-- > 0;) {
+        FxBlock& T = blocks[t];
+        uint64_t touched = 0, win = 0;
+        for (int k : T.idx) touched |= op_bits(ops[k]);
+        if (!(touched & bits)) continue;
+        for (int j = 0; j < T.G; ++j) win |= uint64_t(1) << T.order[j];
+        if (T.shape != FXB_TENSOR || (bits & ~win)) break;
+        T.idx.push_back(i);
+        gone = tx_prepare(n, ops, T, tp, false) == QF_OK;
+        if (!gone) T.idx.pop_back();
+        break;
+      }
+    }
+    if (gone) continue;
+    if (kept != b) blocks[kept] = std::move(blocks[b]);
+    ++kept;
+  }
+  blocks.resize(kept);
+}
+
 }  // namespace
 
 // The passes to run.  Blocks the tensor-core pass takes stay whole, the
@@ -1718,6 +1829,7 @@ std::vector<FxBlock> fx_plan_final(std::vector<HostOp>& ops, int n, int& fusion_
     plan_tensor_block(ops, n, B, pending, out, fusion_k);
   }
   emit_phases(ops, pending, everything, out);
+  if (fusion_k > 1) absorb_channels(ops, n, out);
   return out;
 }
 

@@ -33,8 +33,9 @@
 //    exact and so is a float-to-integer conversion by the 1.5 * 2^23
 //    addition trick;
 //  * Z = A.G / 2^63 = sum acc_delta 2^(49 - 8 delta) (two's complement
-//    int64; |Z| <= 2^62.5 because U is unitary), converted to FP64 once,
-//    exactly rounded, and scaled by 2^(E - 1082).
+//    int64; |Z| <= 2^62.5 because U's norm is at most 1), converted to FP64
+//    once, exactly rounded, and scaled by 2^(E - 1082).  A window that also
+//    takes noise channels (norm at most 2) holds U halved: 2^(E - 1081).
 //
 // Error per output, relative to the row's largest part: the truncation of
 // the inputs (each below 2^-59 of it; through a unit row of U at most
@@ -422,7 +423,7 @@ QF_D void tx_issue(uint32_t abase, uint32_t bbase, uint32_t acc) {
 // arrival on tmem_free), before its last conversions and stores.
 template <bool DB>
 QF_D void tx_epilogue(const TxParams& P, double2* out, uint32_t acc, int E, int64_t b, int oh, uint64_t* tmem_free) {
-  const uint32_t delta = static_cast<uint32_t>(E - 1082) << 20;
+  const uint32_t delta = static_cast<uint32_t>(E - 1082 + P.shift) << 20;
   uint32_t fl = 0u;
   for (int s = 0; s < P.nout; ++s)
     if ((static_cast<uint64_t>(b) & P.out_mout[s]) == P.out_mout[s]) fl ^= P.out_rmask[s];
