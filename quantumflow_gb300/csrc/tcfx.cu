@@ -22,16 +22,21 @@
 //  * both are written in base 256 with balanced digits: X + 0x8080..80 =
 //    sum_t (d_t + 128) 256^(7-t), d_t in [-128, 127] (the amplitudes'
 //    top byte is biased by 0x40 instead, which keeps it below 0x80), so a
-//    byte of the biased integer is a digit (one byte permute per digit
-//    pair) and every digit is exact in fp16;
+//    byte of the biased integer is a digit.  U's digits go in as fp16
+//    integers.  The amplitudes' go in with their bias, each byte as the fp16
+//    subnormal byte 2^-24 (one byte permute per digit pair); what the biases
+//    add to a sum, sum_t bias_t sum_k g_u, depends on U alone and is taken
+//    off the value that the accumulators start from;
 //  * A.G = sum_delta acc_delta 256^(14 - delta), acc_delta = sum over the
 //    digit pairs t + u = delta of the digit GEMMs; delta = 0..7 are kept
 //    (36 of the 64 digit products).  With K = 32 terms per output every
 //    acc_delta is an integer below 2^22 (the top digits are small:
 //    |d_0(A)| <= 33, |d_0(G)| <= 65; the largest, acc_7, is at most
 //    32 (33 128 + 6 128^2 + 128 65) < 2^21.8), so the FP32 accumulation is
-//    exact and so is a float-to-integer conversion by the 1.5 * 2^23
-//    addition trick;
+//    exact (in units of 2^-24), also on top of the 0.75 the accumulators start
+//    from, with which their bit patterns are integers.  A partial sum holds
+//    d_t g_u of the products done and -bias_t g_u of the others, both at
+//    most 128 |g_u|: it keeps the bound of the whole sum in any order;
 //  * Z = A.G / 2^63 = sum acc_delta 2^(49 - 8 delta) (two's complement
 //    int64; |Z| <= 2^62.5 because U's norm is at most 1), converted to FP64
 //    once, exactly rounded, and scaled by 2^(E - 1082).  A window that also
@@ -87,9 +92,48 @@ constexpr uint64_t TX_BIAS = 0x8080808080808080ull;
 constexpr uint64_t TX_BIAS_A = 0x4080808080808080ull;
 constexpr uint32_t TX_A_CHUNK = TX_ROWS * 128;         // 64 fp16 of K per row, 128-byte rows
 constexpr uint32_t TX_A_BYTES = 4 * TX_A_CHUNK;        // 8 digits x 32 reals = 256 K per row
-constexpr uint32_t TX_B_BYTES = TX_ND * TX_KD * 128;   // 256 N-rows, 32 K used of each 128-byte row
-constexpr float TX_MAGIC = 12582912.0f;  // 1.5 * 2^23
-constexpr int32_t TX_MAGIC_BITS = 0x4B400000;
+constexpr uint32_t TX_B_BYTES = TX_ND * TX_KD * 128;   // 256 N-rows of 128 bytes: K = 0 .. 31 digits, then constants
+// An accumulator is 0.75 + e_delta 2^-24 + acc 2^-24, |acc + e_delta| < 2^22: FP32
+// spacing there is 2^-24, so its bits are TX_MAGIC_BITS + e_delta + acc.  The
+// e_delta cancel what the magic bits add to Z (tx_combine).
+constexpr int32_t TX_MAGIC_BITS = 0x3F400000;
+struct TxStart {
+  int32_t e[8];
+};
+constexpr TxStart tx_start() {
+  // Z's share of the magic bits is C = (K2 << 41) + (K2 << 25) + (K2 << 9) +
+  // (K2 >> 7); -C / 2^9 = E0 2^32 + E1 2^16 + E2 mod 2^55, E_j = 256 e_2j + e_2j+1
+  const uint64_t K2 = static_cast<uint32_t>(TX_MAGIC_BITS) * 257u;
+  const uint64_t C = (K2 << 41) + (K2 << 25) + (K2 << 9) + (K2 >> 7);
+  uint64_t v = (uint64_t(0) - C) >> 9;  // 55 bits
+  TxStart t{};
+  int64_t E[3] = {0, 0, 0};
+  for (int j = 2; j >= 0; --j) {
+    const int bits = j == 0 ? 23 : 16;
+    const int64_t low = static_cast<int64_t>(v & ((uint64_t(1) << bits) - 1));
+    E[j] = low >= (int64_t(1) << (bits - 1)) ? low - (int64_t(1) << bits) : low;
+    v = (v - static_cast<uint64_t>(E[j])) >> bits;
+  }
+  for (int j = 0; j < 3; ++j) {
+    const int64_t lo = ((E[j] + 128) & 255) - 128;
+    t.e[2 * j] = static_cast<int32_t>((E[j] - lo) / 256);
+    t.e[2 * j + 1] = static_cast<int32_t>(lo);
+  }
+  return t;
+}
+constexpr TxStart TX_START = tx_start();
+static_assert(((static_cast<uint32_t>(TX_MAGIC_BITS) * 257u) >> 7) % 512u == 0u, "C is a multiple of 2^9");
+constexpr bool tx_start_ok() {
+  uint64_t z = 0;
+  const uint32_t K2 = static_cast<uint32_t>(TX_MAGIC_BITS) * 257u;
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t k = K2 + static_cast<uint32_t>(256 * TX_START.e[2 * j] + TX_START.e[2 * j + 1]);
+    z += j < 3 ? static_cast<uint64_t>(k) << (41 - 16 * j) : static_cast<uint64_t>(k >> 7);
+    if (TX_START.e[2 * j] > 20000 || TX_START.e[2 * j] < -20000) return false;
+  }
+  return z == 0;
+}
+static_assert(tx_start_ok(), "the start values cancel the magic bits");
 
 QF_D uint32_t tx_smem(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -220,52 +264,39 @@ QF_D uint32_t tx_digit_pair(uint64_t x, uint64_t y) {
   return *reinterpret_cast<uint32_t*>(&r);
 }
 
-// The same fp16x2 digit word for the amplitudes (biased by TX_BIAS_A).
-// Digits 0-3 (the high words): one byte permute puts the digit bytes in
-// the low byte of each half and zeros above them (sign copies of the top
-// byte), i.e. the fp16 subnormals byte * 2^-24; two exact half-precision
-// multiply-adds make them byte - bias, leaving the integer ALU (the
-// busiest unit) one instruction per word.  Digits 4-7 as tx_digit_pair.
+// The digit word of the amplitudes (biased by TX_BIAS_A): byte T of x and y
+// in the low byte of each half and zero above, i.e. the fp16 subnormals
+// byte * 2^-24.  Digits 0-3 (the high words): the upper bytes are sign
+// copies of the word's top byte, which is below 0x80.
 template <int T>
 QF_D uint32_t tx_digit_pair_a(uint64_t x, uint64_t y) {
+  constexpr uint32_t b = T < 4 ? 3 - T : 7 - T;  // byte of the high or low word
   if constexpr (T >= 4) {
-    return tx_digit_pair<T>(x, y);
+    return __byte_perm(static_cast<uint32_t>(x), static_cast<uint32_t>(y), b | ((4u + b) << 8)) & 0x00FF00FFu;
   } else {
-    constexpr uint32_t b = 3 - T;  // byte of the high word
     const uint32_t xw = static_cast<uint32_t>(x >> 32), yw = static_cast<uint32_t>(y >> 32);
     // result bytes: byte b of xw, sign of byte 3 of xw, byte b of yw, sign of byte 3 of yw
     // (prmt's sign-replicating selectors: the __byte_perm intrinsic takes
     // only the byte index bits of each selector)
     uint32_t w;
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(xw), "r"(yw), "r"(b | (0xBu << 4) | ((4u + b) << 8) | (0xFu << 12)));
-    constexpr float bias = T == 0 ? 64.f : 128.f;
-    __half2 h = *reinterpret_cast<const __half2*>(&w);
-    const __half2 k = __float2half2_rn(4096.f);
-    h = __hfma2(__hmul2(h, k), k, __float2half2_rn(-bias));
-    return *reinterpret_cast<uint32_t*>(&h);
+    return w;
   }
 }
 
 // Z = sum_delta acc_delta 2^(49 - 8 delta) (= A.G / 2^63) from the eight
-// accumulator words (FP32 integers below 2^22): each becomes 1.5 * 2^23 +
-// acc exactly, whose bit pattern is TX_MAGIC_BITS + acc.  A pair joins in
-// uint32 as b_2j 256 + b_2j+1 = p_j + K2 with p_j = acc_2j 256 + acc_2j+1
-// (|p_j| < 2^30 + 2^22) and K2 = 257 TX_MAGIC_BITS mod 2^32 = 0x8B400000,
-// which never wraps; K2 is a multiple of 128, so the biases of the four
-// pairs leave one constant, subtracted once.  The shifts and adds are
-// multiply-adds (the FMA pipe), the integer ALU being the busiest unit.
-QF_D int64_t tx_combine(const uint32_t (&w)[8]) {
-  uint32_t b[8];
-#pragma unroll
-  for (int d = 0; d < 8; ++d) b[d] = __float_as_uint(__uint_as_float(w[d]) + TX_MAGIC);
-  constexpr uint32_t K2 = static_cast<uint32_t>(TX_MAGIC_BITS) * 257u;
-  static_assert(K2 == 0x8B400000u && K2 % 128u == 0u, "pair bias");
-  constexpr uint64_t C = (static_cast<uint64_t>(K2) << 41) + (static_cast<uint64_t>(K2) << 25) +
-                         (static_cast<uint64_t>(K2) << 9) + (K2 >> 7);
+// accumulator words b = TX_MAGIC_BITS + e_delta + acc.  A pair joins in
+// uint32 as b_2j 256 + b_2j+1 = p_j + K2 + E_j with p_j = acc_2j 256 +
+// acc_2j+1 (|p_j| < 2^30 + 2^22) and K2 = 257 TX_MAGIC_BITS mod 2^32 =
+// 0x7F400000, which never wraps where it matters; K2 is a multiple of 128 and
+// E_3 is 0, so the shift drops what it would drop of p_3, and the rest of the
+// constants cancels (TX_START).  The shifts and adds are multiply-adds (the
+// FMA pipe), the integer ALU being the busiest unit.
+QF_D int64_t tx_combine(const uint32_t (&b)[8]) {
   const uint32_t q0 = b[0] * 256u + b[1], q1 = b[2] * 256u + b[3];
   const uint32_t q2 = b[4] * 256u + b[5], q3 = b[6] * 256u + b[7];
   // sums wrap mod 2^64; the true Z fits int64
-  uint64_t z = fx_madu(q2, 1u << 9, static_cast<uint64_t>(q3 >> 7) - C);
+  uint64_t z = fx_madu(q2, 1u << 9, static_cast<uint64_t>(q3 >> 7));
   z = fx_madu(q1, 1u << 25, z);
   const uint32_t zh = static_cast<uint32_t>(z >> 32) + q0 * 512u;
   return static_cast<int64_t>((static_cast<uint64_t>(zh) << 32) | static_cast<uint32_t>(z));
@@ -296,6 +327,49 @@ QF_D void tx_build_digit(unsigned char* sb, int r, int c, int p, uint64_t x, uin
   const int row = 32 * U + 2 * r + p, k = 2 * c;  // fp16 element k, k + 1 of the row
   *reinterpret_cast<uint32_t*>(sb + tx_piece(row, k >> 3) + (k & 7) * 2) = tx_digit_pair<U>(x, y);
 }
+QF_D uint32_t tx_half2(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// What the accumulators of output real o start from, column block delta:
+// 0.75 + (e_delta - sum_t bias_t sum_k g_(delta - t)) 2^-24, as a sum of
+// products of fp16 numbers with the constant A operand.  The 16 lanes of a
+// half warp hold the 32 biased integers x, y of the row; lane delta of the
+// first eight writes block delta.
+QF_D void tx_build_start(unsigned char* sb, int o, int c, uint64_t x, uint64_t y) {
+  uint32_t s[4];  // sums of the digits 0 and 2, 1 and 3, 4 and 6, 5 and 7 in halves
+  constexpr uint32_t M = 0x00FF00FFu;
+  const uint32_t xh = static_cast<uint32_t>(x >> 32), xl = static_cast<uint32_t>(x);
+  const uint32_t yh = static_cast<uint32_t>(y >> 32), yl = static_cast<uint32_t>(y);
+  s[0] = ((xh >> 8) & M) + ((yh >> 8) & M);
+  s[1] = (xh & M) + (yh & M);
+  s[2] = ((xl >> 8) & M) + ((yl >> 8) & M);
+  s[3] = (xl & M) + (yl & M);
+#pragma unroll
+  for (int d = 1; d < 16; d <<= 1)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], d);
+  if (c >= TX_ND) return;
+  constexpr TxStart start = tx_start();
+  int S = 0, D = 0;
+#pragma unroll
+  for (int u = 0; u < TX_ND; ++u) {
+    const uint32_t w = s[2 * (u >> 2) + (u & 1)];
+    const int sum = static_cast<int>((u & 2) ? w & 0xFFFFu : w >> 16) - 128 * TX_KD;
+    if (u < c) S += 128 * sum;
+    if (u == c) {
+      S += 64 * sum;
+      D = start.e[u];
+    }
+  }
+  D -= S;
+  const int d0 = ((D + 128) & 255) - 128, D1 = (D - d0) >> 8;
+  const int d1 = ((D1 + 128) & 255) - 128, d2 = (D1 - d1) >> 8;
+  const int row = 32 * c + o;
+  *reinterpret_cast<uint4*>(sb + tx_piece(row, 6)) =
+      make_uint4(tx_half2(0.5f, 0.5f), tx_half2(0.5f, d0 * 0x1p-12f), tx_half2(d1 * 0x1p-8f, d2 * 0x1p-4f), 0u);
+  *reinterpret_cast<uint4*>(sb + tx_piece(row, 7)) = make_uint4(0u, 0u, 0u, 0u);
+}
 QF_D void tx_build_b(const TxParams& P, unsigned char* sb, int tid, int nthreads) {
   for (int w = tid; w < 16 * 16 * 2; w += nthreads) {
     const int c = w & 15, p = (w >> 4) & 1, r = w >> 5;
@@ -311,7 +385,14 @@ QF_D void tx_build_b(const TxParams& P, unsigned char* sb, int tid, int nthreads
     tx_build_digit<5>(sb, r, c, p, x, y);
     tx_build_digit<6>(sb, r, c, p, x, y);
     tx_build_digit<7>(sb, r, c, p, x, y);
+    tx_build_start(sb, 2 * r + p, c, x, y);  // whole warps: 512 is a multiple of 32
   }
+  // K = 32 .. 47 of rows 0 .. 127: the constant A operand of tx_issue's first
+  // MMA; its B operand is K = 48 .. 63 (tx_build_start)
+  for (int w = tid; w < TX_ROWS * 2; w += nthreads)
+    *reinterpret_cast<uint4*>(sb + tx_piece(w >> 1, 4 + (w & 1))) =
+        (w & 1) ? make_uint4(0u, 0u, 0u, 0u)
+                : make_uint4(tx_half2(0.5f, 0.5f), tx_half2(0.5f, 0x1p-12f), tx_half2(0x1p-8f, 0x1p-4f), 0u);
 }
 
 // Global index of a row with its window bits zero: the row index's bits
@@ -323,6 +404,13 @@ QF_D int64_t tx_spread(const TxParams& P, int64_t x) {
   return x;
 }
 
+
+// The amplitude boff bytes on: one 64-bit add on the group's address, where
+// an index costs two ORs and a scaled add (n = 28, a pass: 1811 -> 1748 us).
+template <typename T>
+QF_D T* tx_at(T* p, int64_t boff) {
+  return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(p) + static_cast<uintptr_t>(boff));
+}
 
 // Row exponent shared by the AP-amplitude groups of one row (lanes l, l ^ 8
 // and, for AP = 4, l ^ 16, l ^ 24): the largest FP64 exponent field (4095
@@ -374,7 +462,7 @@ QF_D void tx_convert(const TxParams& P, const double2* __restrict__ in, double2 
     }
     if (nb >= 0) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) x[j0 + j] = in[nb | P.off[j0 + j]];
+      for (int j = 0; j < 4; ++j) x[j0 + j] = *tx_at(in + nb, P.boff[j0 + j]);
     }
     // digit t of amplitudes c = AP q + j0 .. + 3: fp16 elements (t & 1) 32 + 2c
     // of chunk t >> 1, one 16-byte piece
@@ -401,8 +489,17 @@ QF_D void tx_convert(const TxParams& P, const double2* __restrict__ in, double2 
 }
 
 // The MMAs of one tile: amplitude digit t against gate digits 0 .. 7 - t,
-// into accumulator columns [acc + 32 t, acc + 256)
+// into accumulator columns [acc + 32 t, acc + 256).  Before them one MMA of
+// B's constant columns sets every accumulator to its start value, where FP32
+// has the spacing of the sums' unit: the words read back are integers
+// without an addition per accumulator in the epilogue, and the amplitudes'
+// digits need no conversion from their biased bytes: 21% fewer instructions
+// (n = 28, a pass: 1748 -> 1695 us, 0.76 of the copy rate; n = 24: 118 -> 114).
+// What bounds the pass is then the latency of its loads, one tile in flight a
+// CTA; loads two tiles ahead through shared memory or registers, and
+// prefetches into L2, ran slower at n <= 22 or at every size.
 QF_D void tx_issue(uint32_t abase, uint32_t bbase, uint32_t acc) {
+  tx_mma(acc, tx_desc(bbase + 64u), tx_desc(bbase + 96u), tx_idesc(TX_KD * TX_ND), 0u);
 #pragma unroll
   for (int t = 0; t < TX_ND; ++t) {
     const uint32_t idesc = tx_idesc(TX_KD * (TX_ND - t));
@@ -410,7 +507,7 @@ QF_D void tx_issue(uint32_t abase, uint32_t bbase, uint32_t acc) {
     for (int ks = 0; ks < 2; ++ks) {
       const uint32_t a = abase + (t >> 1) * TX_A_CHUNK + (t & 1) * 64 + ks * 32;
       const uint32_t b = bbase + ks * 32;
-      tx_mma(acc + static_cast<uint32_t>(TX_KD * t), tx_desc(a), tx_desc(b), idesc, (t > 0 || ks > 0) ? 1u : 0u);
+      tx_mma(acc + static_cast<uint32_t>(TX_KD * t), tx_desc(a), tx_desc(b), idesc, 1u);
     }
   }
 }
@@ -458,7 +555,7 @@ QF_D void tx_epilogue(const TxParams& P, double2* out, uint32_t acc, int E, int6
         wi[d] = a4[DB ? (q & 1) : 0][d][2 * a + 1];
       }
       const uint32_t ds = delta ^ (((fl >> j) & 1u) << 31);
-      out[b | P.off[j]] = make_double2(tx_out(tx_combine(wr), ds), tx_out(tx_combine(wi), ds));
+      *tx_at(out + b, P.boff[j]) = make_double2(tx_out(tx_combine(wr), ds), tx_out(tx_combine(wi), ds));
     }
   }
 }
@@ -493,7 +590,7 @@ struct TxShape {
 // Register split (AP = 8: 640 threads launched at 96 registers, 61440 in
 // all): the issuer's warpgroup gives its registers up (24 each), the
 // converters take 120 and the epilogue 104: 256 x 120 + 256 x 104 + 128 x 24
-// = 60416 (at N=28, 128 / 96 ran 1.5% and 112 / 112 0.7% slower).
+// = 60416 (at N=28, 128 / 96 and 112 / 112 run within 0.4% of it).
 constexpr int TX_REG_LAUNCH = 96, TX_REG_CONV = 120, TX_REG_EPI = 104, TX_REG_ISSUE = 24;
 static_assert(256 * TX_REG_CONV + 256 * TX_REG_EPI + 128 * TX_REG_ISSUE <= 640 * TX_REG_LAUNCH,
               "register split above the launch's registers");
@@ -551,7 +648,7 @@ __global__ void __launch_bounds__(TxShape<AP>::THREADS, 1) k_txpipe(const __grid
     if (tile < ntiles) {
       const int64_t b = tx_spread(P, tile * TX_ROWS) | grow;
 #pragma unroll
-      for (int j = 0; j < AP; ++j) x[j] = in[b | P.off[j]];
+      for (int j = 0; j < AP; ++j) x[j] = *tx_at(in + b, P.boff[j]);
     }
     int a = 0, ar = 0;  // A stage (it % 3) and its round (it / 3)
     for (int it = 0; tile < ntiles; tile += step, ++it) {
