@@ -472,43 +472,69 @@ __global__ void __launch_bounds__(SCAN_CHUNK) k_scan_offsets(double* totals, con
   if (i < nblocks) totals[i] = carry + incl[i] - totals[i];
 }
 
-// The sequential sums: one scan block per lane, 32 of them per warp, staged
-// through shared memory in columns of 32 amplitudes (loads and stores stay
-// contiguous; row stride 33 keeps the lanes on distinct banks).  The chain
-// of 1024 dependent FP64 adds is the bound; 32 chains share each issue.
-// n = 22: 311 -> 84 us (one thread of each 256-thread block summed).
-__global__ void __launch_bounds__(32) k_scan_blocks(double* p, int64_t namps, const double* offsets,
-                                                    int64_t nblocks) {
-  __shared__ double sh[32][33];
-  const int lane = threadIdx.x;
+// The sequential sums: one scan block per lane of warp 0, 32 of them per
+// CTA, in tiles of 64 columns in shared memory (a row stride of 65 keeps the
+// lanes on distinct banks).  While warp 0 sums a tile, the other warps
+// write the sums before it back and bring the next tile in.  The chain of
+// 1024 dependent FP64 adds is the bound, about 60 ns each; 32 chains share
+// each issue of the FP64 pipe.  A draw of 1000 outcomes, all kernels: n = 22
+// 123 us (387 with one thread of a block per 1024 amplitudes summing), n = 24
+// 291 (1362), n = 16 87 (85), n = 8 39 (81).  With one warp moving the data
+// and summing it, read-outs below n = 20 were 35 us slower than this.
+constexpr int SCAN_COLS = 64;
+__global__ void __launch_bounds__(256) k_scan_blocks(double* p, int64_t namps, const double* offsets,
+                                                     int64_t nblocks) {
+  __shared__ double sh[2][32][SCAN_COLS + 1];
+  constexpr int ITEMS = 32 * SCAN_COLS, MOVERS = 224, PER = (ITEMS + MOVERS - 1) / MOVERS;
+  const int lane = threadIdx.x & 31;
   const int64_t b0 = (int64_t)blockIdx.x * 32;
-  double c = b0 + lane < nblocks ? offsets[b0 + lane] : 0.0;
-  double v[32];
-  auto load = [&](int col) {
+  const int cols = namps < SCAN_BLOCK ? (int)namps : SCAN_BLOCK;
+  const int tiles = (cols + SCAN_COLS - 1) / SCAN_COLS;
+  auto at = [&](int tile, int i) { return (b0 + i / SCAN_COLS) * SCAN_BLOCK + tile * SCAN_COLS + i % SCAN_COLS; };
+  for (int i = threadIdx.x; i < ITEMS; i += 256) {
+    const int64_t x = at(0, i);
+    sh[0][i / SCAN_COLS][i % SCAN_COLS] = x < namps ? p[x] : 0.0;
+  }
+  double c = threadIdx.x < 32 && b0 + lane < nblocks ? offsets[b0 + lane] : 0.0;
+  __syncthreads();
+  for (int k = 0; k <= tiles; ++k) {
+    if (threadIdx.x < 32) {
+      if (k < tiles) {
+        double* row = sh[k & 1][lane];
 #pragma unroll
-    for (int r = 0; r < 32; ++r) {
-      const int64_t x = (b0 + r) * SCAN_BLOCK + col + lane;
-      v[r] = x < namps ? p[x] : 0.0;
+        for (int j0 = 0; j0 < SCAN_COLS; j0 += 16) {
+          double v[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = row[j0 + j];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            c += v[j];
+            row[j0 + j] = c;
+          }
+        }
+      }
+    } else {  // a thread's items stay its own, so a buffer is written after it is read
+      const int t = threadIdx.x - 32;
+      double v[PER];
+#pragma unroll
+      for (int m = 0; m < PER; ++m) {
+        const int i = t + m * MOVERS;
+        const int64_t x = at(k + 1, i);
+        v[m] = i < ITEMS && k + 1 < tiles && x < namps ? p[x] : 0.0;
+      }
+#pragma unroll
+      for (int m = 0; m < PER; ++m) {
+        const int i = t + m * MOVERS;
+        if (i >= ITEMS) break;
+        double& slot = sh[(k + 1) & 1][i / SCAN_COLS][i % SCAN_COLS];
+        if (k > 0) {
+          const int64_t x = at(k - 1, i);
+          if (x < namps) p[x] = slot;
+        }
+        if (k + 1 < tiles) slot = v[m];
+      }
     }
-  };
-  load(0);
-  for (int col = 0; col < SCAN_BLOCK; col += 32) {
-#pragma unroll
-    for (int r = 0; r < 32; ++r) sh[r][lane] = v[r];
-    __syncwarp();
-    if (col + 32 < SCAN_BLOCK) load(col + 32);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      c += sh[lane][j];
-      sh[lane][j] = c;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < 32; ++r) {
-      const int64_t x = (b0 + r) * SCAN_BLOCK + col + lane;
-      if (x < namps) p[x] = sh[r][lane];
-    }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
@@ -572,7 +598,7 @@ static int sample_cdf(const void* psi, int n, int layout, void* ws, double* scra
   }
   k_scan_chunks<<<(unsigned)nc, SCAN_CHUNK, 0, stream>>>(totals, scratch, scratch + nb, nb);
   k_scan_offsets<<<(unsigned)nc, SCAN_CHUNK, 0, stream>>>(totals, scratch, scratch + nb, nb);
-  k_scan_blocks<<<(unsigned)((nb + 31) / 32), 32, 0, stream>>>(cdf, namps, totals, nb);
+  k_scan_blocks<<<(unsigned)((nb + 31) / 32), 256, 0, stream>>>(cdf, namps, totals, nb);
   return check_cuda(cudaGetLastError());
 }
 
