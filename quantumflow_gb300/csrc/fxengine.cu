@@ -751,7 +751,7 @@ bool is_swap(const HostOp& op) {
 // tensor-core passes) the group kernel's limits on element-wise ops do not
 // apply, 3- and 4-qubit unitary gates become blocks of their own, and so do
 // runs of at least three disjoint SWAPs: one exchange pass (n = 23: 70 us)
-// against one tensor-core pass (69 us) per two of them.  Where the list has
+// against one tensor-core pass (59 us) per two of them.  Where the list has
 // channels a pass can take (tx_channel), a dense gate and its image on the
 // bits a constant distance away (the ket and bra sides of a density) stay in
 // one window, which then takes the channels on those qubits: two layers with
@@ -1198,7 +1198,6 @@ inline Dd dd_mul_d(Dd a, double b) {
 struct Cdd {
   Dd re, im;
 };
-inline bool cdd_zero(const Cdd& v) { return v.re.hi == 0.0 && v.im.hi == 0.0; }
 // g * v for an FP64 complex g
 inline Cdd cdd_mul(cplx g, const Cdd& v) {
   return {dd_add(dd_mul_d(v.re, g.real()), dd_neg(dd_mul_d(v.im, g.imag()))),
@@ -1747,11 +1746,11 @@ void plan_tensor_block(const std::vector<HostOp>& ops, int n, const FxBlock& who
 // its bits when that pass's window has them all and the passes between do
 // not touch them: the pass costs the same, and the sweep of its own goes
 // (n = 22: 36 us for a depolarizing channel, 23 for a dephasing one, beside
-// 31 for the pass).  Two layers with a channel per qubit, 11 qubits: 1065 ->
+// 30 for the pass).  Two layers with a channel per qubit, 11 qubits: 1065 ->
 // 665 us a call; 8 qubits, error against 80-bit
 // arithmetic 4.4e-16 -> 3.7e-16.  Never a pass of channels alone: it would
 // hold their rows to a shared exponent that no gate asks for, and gain little
-// (31 us against two sweeps).
+// (30 us against two sweeps).
 void absorb_channels(const std::vector<HostOp>& ops, int n, std::vector<FxBlock>& blocks) {
   static thread_local TxParams tp;
   size_t kept = 0;
