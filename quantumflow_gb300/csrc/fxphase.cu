@@ -20,9 +20,10 @@
 // Arithmetic: an amplitude's two parts share one exponent (57-bit integers,
 // fx.cuh), phases are 2^58 integers multiplied with 2^-57 relative error, and
 // each part is rounded to FP64 once by the exactly rounding convert.
-// Bound: HBM (32 bytes an amplitude) beside about 120 instructions.  QFT,
-// n = 23: 73 us a pass (0.27 GB moved; 40 us at the copy rate); the interpreted group passes
-// took 950 to 1570 us.
+// Bound: about 220 instructions an amplitude (n = 24: issue 58%, integer ALU
+// 60%), then HBM (32 bytes an amplitude).  QFT, n = 23: 70 us a pass (0.27 GB
+// moved; 40 us at the copy rate); the interpreted group passes took 950 to
+// 1570 us.
 #include <atomic>
 
 #include "fx.cuh"
@@ -82,8 +83,34 @@ QF_D double2 fxp_flip(double2 v, uint32_t flip) {
                       fx_double(fx_hiword(v.y) ^ flip, fx_loword(v.y)));
 }
 
-template <int G, typename IT>
-__global__ void __launch_bounds__(FXP_THREADS, 2) k_fxphase(const __grid_constant__ FxPhaseParams P, int nch) {
+// The kernels below read only parameters up to here, so they may run while the
+// previous pass of the stream drains (programmatic dependent launch); nothing
+// of the state is touched before that pass has finished.  QFT, n = 16:
+// 72 -> 61 us, n = 20: 147 -> 135, n = 23: 847 -> 823.
+QF_D void fxp_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename P, typename... A>
+int fxp_launch(void (*kernel)(P, A...), int64_t grid, int threads, size_t smem, cudaStream_t stream, const P& params,
+               A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kernel, params, args...));
+}
+
+// CTAS of them share an SM: two load eight amplitudes of a thread at a time;
+// three, at fewer registers, load four.
+template <int G, typename IT, int CTAS>
+__global__ void __launch_bounds__(FXP_THREADS, CTAS) k_fxphase(const __grid_constant__ FxPhaseParams P, int nch) {
   extern __shared__ __align__(16) longlong2 tab[];  // [1 + nch][G + 1][256]
   constexpr int F = G + 1, TS = 1 << FXP_LOW;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -105,6 +132,7 @@ __global__ void __launch_bounds__(FXP_THREADS, 2) k_fxphase(const __grid_constan
     }
   }
   __syncthreads();
+  fxp_wait();
   const IT ngroups = IT(1) << tbits;
   const IT ntiles = (ngroups + FXP_THREADS - 1) / FXP_THREADS;
   for (IT tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -143,8 +171,8 @@ __global__ void __launch_bounds__(FXP_THREADS, 2) k_fxphase(const __grid_constan
       inner[3] = fxp_mul(fn[0], fn[1]);
     }
 #pragma unroll
-    for (int o0 = 0; o0 < NO; o0 += 2) {
-      constexpr int STEP = NO < 2 ? 1 : 2;
+    for (int o0 = 0; o0 < NO; o0 += CTAS > 2 ? 1 : 2) {
+      constexpr int STEP = NO < 2 || CTAS > 2 ? 1 : 2;
       double2 x[STEP * NI];
 #pragma unroll
       for (int k = 0; k < STEP * NI; ++k) x[k] = P.in[xb | (IT)P.off[o0 * NI + k]];
@@ -184,7 +212,7 @@ __global__ void __launch_bounds__(FXP_THREADS, 2) k_fxphase(const __grid_constan
   }
 }
 
-template <int G, typename IT>
+template <int G, typename IT, int CTAS>
 int phase_launch_t(const FxPhaseParams& P, cudaStream_t stream) {
   const int hbits = P.n - G - FXP_LOW;
   const int nch = hbits <= 0 ? 0 : (hbits + FXP_LOW - 1) / FXP_LOW;
@@ -193,16 +221,15 @@ int phase_launch_t(const FxPhaseParams& P, cudaStream_t stream) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!attr_set[dev].load()) {  // up to four tables (n <= 34): 100 KiB
-    int rc = check_cuda(cudaFuncSetAttribute(k_fxphase<G, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    int rc = check_cuda(cudaFuncSetAttribute(k_fxphase<G, IT, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              5 * (G + 1) * (16 << FXP_LOW)));
     if (rc) return rc;
     attr_set[dev].store(1);
   }
   int64_t grid = hbits <= 0 ? 1 : int64_t(1) << hbits;
-  const int64_t cap = (int64_t)device_sm_count() * 2;
+  const int64_t cap = (int64_t)device_sm_count() * CTAS;
   if (grid > cap) grid = cap;
-  k_fxphase<G, IT><<<(int)grid, FXP_THREADS, smem, stream>>>(P, nch);
-  return check_cuda(cudaGetLastError());
+  return fxp_launch(k_fxphase<G, IT, CTAS>, grid, FXP_THREADS, smem, stream, P, nch);
 }
 
 // A CTA exchanges the tiles at base b and pi(b) (the tile bits include the
@@ -232,6 +259,7 @@ __global__ void __launch_bounds__(FXSW_THREADS) k_fxswap(const __grid_constant__
       }
   }
   const int64_t nbase = int64_t(1) << (P.n - P.nt);
+  fxp_wait();
   for (int64_t u = blockIdx.x; u < nbase; u += gridDim.x) {
     int64_t b = u;
     for (int j = 0; j < P.nt; ++j) b = insert0(b, (int)P.tb[j]);
@@ -264,14 +292,23 @@ __global__ void __launch_bounds__(FXSW_THREADS) k_fxswap(const __grid_constant__
 
 }  // namespace
 
+// Three CTAs an SM from 2^11 tiles of 256 threads (five rounds of them) on,
+// where they hide more of each other's latency: QFT, n = 24 1595 -> 1560 us,
+// n = 26 6731 -> 6530; below, the last round is emptier than with two: n = 21
+// 249 with two, 265 with three.
+template <int G>
+static int phase_launch(const FxPhaseParams& P, cudaStream_t stream) {
+  if (P.n > 31) return phase_launch_t<G, int64_t, 3>(P, stream);
+  return P.n - G - FXP_LOW >= 11 ? phase_launch_t<G, uint32_t, 3>(P, stream) : phase_launch_t<G, uint32_t, 2>(P, stream);
+}
+
 int fx_phase_launch(const FxPhaseParams& P, cudaStream_t stream) {
-  const bool w = P.n <= 31;
   switch (P.G) {
-    case 0: return w ? phase_launch_t<0, uint32_t>(P, stream) : phase_launch_t<0, int64_t>(P, stream);
-    case 1: return w ? phase_launch_t<1, uint32_t>(P, stream) : phase_launch_t<1, int64_t>(P, stream);
-    case 2: return w ? phase_launch_t<2, uint32_t>(P, stream) : phase_launch_t<2, int64_t>(P, stream);
-    case 3: return w ? phase_launch_t<3, uint32_t>(P, stream) : phase_launch_t<3, int64_t>(P, stream);
-    case 4: return w ? phase_launch_t<4, uint32_t>(P, stream) : phase_launch_t<4, int64_t>(P, stream);
+    case 0: return phase_launch<0>(P, stream);
+    case 1: return phase_launch<1>(P, stream);
+    case 2: return phase_launch<2>(P, stream);
+    case 3: return phase_launch<3>(P, stream);
+    case 4: return phase_launch<4>(P, stream);
   }
   return QF_ERR_NOT_SUPPORTED;
 }
@@ -280,8 +317,7 @@ int fx_swap_launch(const FxSwapParams& P, cudaStream_t stream) {
   int64_t grid = int64_t(1) << (P.n - P.nt);
   const int64_t cap = (int64_t)device_sm_count() * 6;
   if (grid > cap) grid = cap;
-  k_fxswap<<<(int)grid, FXSW_THREADS, 0, stream>>>(P);
-  return check_cuda(cudaGetLastError());
+  return fxp_launch(k_fxswap, grid, FXSW_THREADS, 0, stream, P);
 }
 
 }  // namespace qf
