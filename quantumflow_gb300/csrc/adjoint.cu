@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(256) k_adj(const __grid_constant__ AdjParams P
     fence_mbar_init();
   }
   __syncthreads();
+  pdl_wait();
 
   auto tile_base = [&](int64_t t) {
     int64_t v = t << P.L;
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(256) k_adjw(const __grid_constant__ AdjWParams
   __shared__ double red[8][4];
   const int necoef = 2 * P.ndiag + P.ncut;
   for (int i = threadIdx.x; i < necoef; i += blockDim.x) scoef[i] = P.coef[i];
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // this warp's ring: [stage][vector][register][lane]
   E* ring = reinterpret_cast<E*>(smem_raw + (((size_t)necoef * sizeof(Coef) + 127) & ~size_t(127))) +
@@ -490,6 +492,7 @@ __global__ void __launch_bounds__(256) k_adjw(const __grid_constant__ AdjWParams
 
 // out[s] = sum over rows of rows[r][s]; one warp per slot, fixed order
 __global__ void k_rows_sum(const double* rows, int nrows, int nslots, double* out) {
+  pdl_wait();
   const int s = blockIdx.x;
   if (s >= nslots) return;
   double v = 0.0;
@@ -560,8 +563,7 @@ int qaoa_wide_grad(void* psi, int n, int layout, const uint16_t* cuts, int nedge
   if (rc) return rc;
   rc = qtile_grad(psi, ws, n, cuts, nedges, p, beta, gamma, rows, nslots, stream);
   if (rc) return rc;
-  k_rows_sum<<<nslots, 32, 0, stream>>>(rows, (int)nrows, nslots, out);
-  return check_cuda(cudaGetLastError());
+  return pdl_launch(k_rows_sum, nslots, 32, 0, stream, rows, (int)nrows, nslots, out);
 }
 
 template <int LAY, int RB>
@@ -577,8 +579,7 @@ static int launch_adjw(AdjWParams& P, int grid, cudaStream_t stream) {
   }
   const size_t necoef = (size_t)(2 * P.ndiag + P.ncut);
   const size_t smem = ((necoef * sizeof(Coef) + 127) & ~size_t(127)) + adjw_ring_bytes<LAY, RB>();
-  k_adjw<LAY, RB><<<grid, 256, smem, stream>>>(P);
-  return check_cuda(cudaGetLastError());
+  return pdl_launch(k_adjw<LAY, RB>, grid, 256, smem, stream, P);
 }
 
 // Warp-tile adjoint sweep (k_adjw); psi holds the forward state.  Per layer
@@ -691,8 +692,7 @@ static int launch_adj(AdjParams& P, int grid, cudaStream_t stream) {
     if (rc) return rc;
     attr[dev].store(true);
   }
-  k_adj<LAY><<<grid, 256, smem, stream>>>(P);
-  return check_cuda(cudaGetLastError());
+  return pdl_launch(k_adj<LAY>, grid, 256, smem, stream, P);
 }
 
 // out[0..p) = d<C>/d gamma, out[p..2p) = d<C>/d beta, out[2p] = <C>.
@@ -718,8 +718,7 @@ int qaoa_grad(void* psi, int n, int layout, const uint16_t* cuts, int nedges, in
     else
       rc = qaoa_grad_warp(psi, n, layout, cuts, nedges, p, beta, gamma, node_theta, lam, rows, nslots, stream);
     if (rc) return rc;
-    k_rows_sum<<<nslots, 32, 0, stream>>>(rows, nrows, nslots, out);
-    return check_cuda(cudaGetLastError());
+    return pdl_launch(k_rows_sum, nslots, 32, 0, stream, rows, nrows, nslots, out);
   }
   const int grid = adj_grid(n, layout);
   int rc = check_cuda(cudaMemsetAsync(rows, 0, (size_t)grid * nslots * sizeof(double), stream));
@@ -854,8 +853,7 @@ int qaoa_grad(void* psi, int n, int layout, const uint16_t* cuts, int nedges, in
   if (p == 0) {  // <C> only
     return reduce_diag(psi, n, layout, 1, cuts, nullptr, out + 2 * p, rows, stream);
   }
-  k_rows_sum<<<nslots, 32, 0, stream>>>(rows, grid, nslots, out);
-  return check_cuda(cudaGetLastError());
+  return pdl_launch(k_rows_sum, nslots, 32, 0, stream, rows, grid, nslots, out);
 }
 
 }  // namespace qf

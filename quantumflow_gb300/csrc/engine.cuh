@@ -358,4 +358,27 @@ int timing_enable(int on);
 int timing_collect(double* ms, int64_t* counts, int nkinds);
 int check_cuda(cudaError_t e);
 
+// Overlapped launches (programmatic dependent launch): a kernel started with
+// pdl_launch may run while the stream's previous kernel drains, up to its
+// pdl_wait, before which it reads parameters only; every thread waits there
+// until that kernel has finished and its writes are visible.
+QF_D void pdl_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+int pdl_launch(void (*kernel)(P...), int64_t grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
 }  // namespace qf

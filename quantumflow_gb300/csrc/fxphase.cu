@@ -83,30 +83,6 @@ QF_D double2 fxp_flip(double2 v, uint32_t flip) {
                       fx_double(fx_hiword(v.y) ^ flip, fx_loword(v.y)));
 }
 
-// The kernels below read only parameters up to here, so they may run while the
-// previous pass of the stream drains (programmatic dependent launch); nothing
-// of the state is touched before that pass has finished.  QFT, n = 16:
-// 72 -> 61 us, n = 20: 147 -> 135, n = 23: 847 -> 823.
-QF_D void fxp_wait() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-template <typename P, typename... A>
-int fxp_launch(void (*kernel)(P, A...), int64_t grid, int threads, size_t smem, cudaStream_t stream, const P& params,
-               A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return check_cuda(cudaLaunchKernelEx(&cfg, kernel, params, args...));
-}
-
 // CTAS of them share an SM: two load eight amplitudes of a thread at a time;
 // three, at fewer registers, load four.
 template <int G, typename IT, int CTAS>
@@ -132,7 +108,7 @@ __global__ void __launch_bounds__(FXP_THREADS, CTAS) k_fxphase(const __grid_cons
     }
   }
   __syncthreads();
-  fxp_wait();
+  pdl_wait();  // QFT, launches overlapped: n = 16 72 -> 61 us, n = 20 147 -> 135, n = 23 847 -> 823
   const IT ngroups = IT(1) << tbits;
   const IT ntiles = (ngroups + FXP_THREADS - 1) / FXP_THREADS;
   for (IT tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -229,7 +205,7 @@ int phase_launch_t(const FxPhaseParams& P, cudaStream_t stream) {
   int64_t grid = hbits <= 0 ? 1 : int64_t(1) << hbits;
   const int64_t cap = (int64_t)device_sm_count() * CTAS;
   if (grid > cap) grid = cap;
-  return fxp_launch(k_fxphase<G, IT, CTAS>, grid, FXP_THREADS, smem, stream, P, nch);
+  return pdl_launch(k_fxphase<G, IT, CTAS>, grid, FXP_THREADS, smem, stream, P, nch);
 }
 
 // A CTA exchanges the tiles at base b and pi(b) (the tile bits include the
@@ -259,7 +235,7 @@ __global__ void __launch_bounds__(FXSW_THREADS) k_fxswap(const __grid_constant__
       }
   }
   const int64_t nbase = int64_t(1) << (P.n - P.nt);
-  fxp_wait();
+  pdl_wait();
   for (int64_t u = blockIdx.x; u < nbase; u += gridDim.x) {
     int64_t b = u;
     for (int j = 0; j < P.nt; ++j) b = insert0(b, (int)P.tb[j]);
@@ -317,7 +293,7 @@ int fx_swap_launch(const FxSwapParams& P, cudaStream_t stream) {
   int64_t grid = int64_t(1) << (P.n - P.nt);
   const int64_t cap = (int64_t)device_sm_count() * 6;
   if (grid > cap) grid = cap;
-  return fxp_launch(k_fxswap, grid, FXSW_THREADS, 0, stream, P);
+  return pdl_launch(k_fxswap, grid, FXSW_THREADS, 0, stream, P);
 }
 
 }  // namespace qf

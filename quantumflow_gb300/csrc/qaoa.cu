@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(256) k_qaoaw(const __grid_constant__ QaoaWPara
   Coef* scoef = reinterpret_cast<Coef*>(smem_raw);
   const int necoef = P.hasB ? 2 * P.ndiag + P.ncut : 0;
   for (int i = threadIdx.x; i < necoef; i += blockDim.x) scoef[i] = P.coef[i];
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   E* ring = reinterpret_cast<E*>(smem_raw + (((size_t)necoef * sizeof(Coef) + 127) & ~size_t(127))) +
             (size_t)warp * QW_STAGES * R * 32;
@@ -208,8 +209,7 @@ static int launch_qw(QaoaWParams& P, cudaStream_t stream) {
   int64_t grid = (nsub + 7) / 8;
   const int64_t cap = (int64_t)device_sm_count() * 4;
   if (grid > cap) grid = cap;
-  k_qaoaw<LAY, RB><<<(int)grid, 256, smem, stream>>>(P);
-  return check_cuda(cudaGetLastError());
+  return pdl_launch(k_qaoaw<LAY, RB>, grid, 256, smem, stream, P);
 }
 
 static int qaoa_state_warp(void* psi, int n, int layout, const uint16_t* cuts, int nedges, int p,

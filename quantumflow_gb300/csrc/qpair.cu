@@ -44,6 +44,7 @@ QF_D unsigned char* qp_table(const QPairParams& P, unsigned char* smem) {
   if (P.F.cost)
     for (int i = threadIdx.x; i < P.ncut; i += blockDim.x) tab[i] = P.coef[i];
   __syncthreads();
+  pdl_wait();
   return smem + ((P.ncut * sizeof(Coef) + 127) & ~size_t(127));
 }
 
@@ -136,8 +137,8 @@ int qpair_state(void* psi, int n, const uint16_t* cuts, int nedges, int p, const
       for (int cv = 0; cv <= nedges; ++cv)
         P.coef[cv] = make_coef(std::polar(1.0, gamma[F.layerB] * (0.5 * nedges - cv)), C64);
     }
-    k_qpair_fwd<<<grid, PairShape<C64, QP_RBF>::NT, qp_smem<QP_RBF>(0, P.ncut), stream>>>(P);
-    if ((rc = check_cuda(cudaGetLastError()))) return rc;
+    rc = pdl_launch(k_qpair_fwd, grid, PairShape<C64, QP_RBF>::NT, qp_smem<QP_RBF>(0, P.ncut), stream, P);
+    if (rc) return rc;
   }
   return QF_OK;
 }
@@ -175,8 +176,8 @@ int qpair_grad(void* psi, void* lam, int n, const uint16_t* cuts, int nedges, in
     P.slot_cut = F.cost ? l : -1;
     P.slot_e = F.init ? 2 * p : -1;
     P.slot_b = F.hasB ? p + l - 1 : -1;
-    k_qpair_adj<<<grid, PairShape<C64, QP_RBA>::NT, qp_smem<QP_RBA>(2, P.ncut), stream>>>(P);
-    if ((rc = check_cuda(cudaGetLastError()))) return rc;
+    rc = pdl_launch(k_qpair_adj, grid, PairShape<C64, QP_RBA>::NT, qp_smem<QP_RBA>(2, P.ncut), stream, P);
+    if (rc) return rc;
   }
   return QF_OK;
 }
