@@ -7,7 +7,7 @@
 // the same order, half of the passes over the state.
 // Bound: HBM (adjoint passes, 106 us at n = 24 of 80 at the copy rate); the
 // forward passes, 66 us of 40, FP32 issue and shuffles at the layer
-// boundaries.  n = 24, p = 6: 4956 -> 3050 us a gradient evaluation
+// boundaries.  n = 24, p = 6: 4967 -> 2960 us a gradient evaluation
 // (forward 25 passes -> 13, adjoint 37 -> 19).
 #include <algorithm>
 #include <atomic>
