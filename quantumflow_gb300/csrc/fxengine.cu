@@ -674,7 +674,8 @@ bool tx_wide(const HostOp& op) {
 //    beside its row's inputs is then no more a difference of large ones
 //    than behind a gate, and the row's shared exponent serves it as well
 //    (a strong damping or a projection keeps the native FP64 kernels);
-//  * |M|_1 |M|_inf, which bounds the square of the 2-norm, is at most 4;
+//  * |M|_1 |M|_inf, which bounds the square of the 2-norm, is below 4, so
+//    that every entry is below 2 and its 2^62 integer fits 64 bits;
 //  * no entry but 0 is below 2^-12, of which the window's 2^-62 grid would
 //    keep fewer than 50 bits.
 double tx_channel(const HostOp& op) {
@@ -686,7 +687,7 @@ double tx_channel(const HostOp& op) {
       if (!(a >= 0.5)) return 0.0;
       big = std::max(big, a);
     }
-    return big <= 2.0 ? big * big : 0.0;
+    return big < 2.0 ? big * big : 0.0;
   }
   if (op.type != OP_DENSE1 && op.type != OP_DENSE2 && !(op.type == OP_DENSEK && op.k <= 4)) return 0.0;
   double row = 0.0, col[16] = {0.0};
@@ -703,7 +704,7 @@ double tx_channel(const HostOp& op) {
     row = std::max(row, d + off);
   }
   const double bound = row * *std::max_element(col, col + D);
-  return bound <= 4.0 ? bound : 0.0;
+  return bound < 4.0 ? bound : 0.0;
 }
 
 constexpr int FX_G_MAX = 4;
