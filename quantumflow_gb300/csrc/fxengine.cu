@@ -709,6 +709,13 @@ double tx_channel(const HostOp& op) {
 
 constexpr int FX_G_MAX = 4;
 
+// Most gates multiplied into one window.  A gate counts as unitary when every
+// entry of U U^H - 1 is within FX_UNIT_TOL, so its norm is at most
+// 1 + 2 FX_UNIT_TOL (4x4), and 256 of them stay below 1 + 2^-20, the bound the
+// pass's digits are laid out for.
+constexpr int TX_MAX_GATES = 256;
+static_assert(TX_MAX_GATES * 2 * FX_UNIT_TOL < 0x1p-20, "norm of a window");
+
 // Greedy passes: element-wise ops join the current pass; a dense op joins
 // while the pass's dense bits stay within gmax; ops the fixed-point kernels
 // do not take close the pass and run alone in native FP64.
@@ -749,8 +756,9 @@ bool is_swap(const HostOp& op) {
 }
 
 // The greedy blocks of the ops `list`.  With `tensor` (planning for the
-// tensor-core passes) the group kernel's limits on element-wise ops do not
-// apply, 3- and 4-qubit unitary gates become blocks of their own, and so do
+// tensor-core passes) a block takes half of TX_MAX_GATES ops, which leaves
+// room for the diagonals waiting for it, instead of what the group kernel's
+// parameters hold; 3- and 4-qubit unitary gates become blocks of their own, and so do
 // runs of at least three disjoint SWAPs: one exchange pass (n = 23: 70 us)
 // against one tensor-core pass (59 us) per two of them.  Where the list has
 // channels a pass can take (tx_channel), a dense gate and its image on the
@@ -827,8 +835,9 @@ std::vector<FxBlock> fx_blocks(const std::vector<HostOp>& ops, const std::vector
                 std::find(add, add + nadd, im.gb[j]) == add + nadd;
     }
     second = first;
-    const bool fits = both <= gmax && (tensor || ((int)cur.idx.size() < FXG_MAX_OPS / 3 &&
-                                                          cur.ncoef + need <= FXG_MAX_COEF));
+    const bool fits = both <= gmax && (tensor ? (int)cur.idx.size() < TX_MAX_GATES / 2
+                                              : (int)cur.idx.size() < FXG_MAX_OPS / 3 &&
+                                                    cur.ncoef + need <= FXG_MAX_COEF);
     if (!cur.idx.empty() && (!fuse || !fits)) close();
     if (kind == FXK_DENSE) {
       for (int j = 0; j < op.k; ++j)
@@ -1330,7 +1339,9 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
     P.boff[c] = 16 * o;
   }
   double norm2 = 1.0;
+  int gates = 0;
   for (int i : B.idx) {
+    if (ops[i].type != OP_SIGN && ++gates > TX_MAX_GATES) return QF_ERR_NOT_SUPPORTED;
     if (fx_kind(ops[i]) != FXK_NATIVE || tx_wide(ops[i])) continue;
     const double b = tx_channel(ops[i]);
     if (b == 0.0) return QF_ERR_NOT_SUPPORTED;
@@ -1429,8 +1440,9 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
     }
   }
   if (!matrix) return QF_OK;
-  // unit rows of a product of gates unitary to 1e-9: well inside the
-  // digits' bounds (|G| < 2^62.9 keeps G + bias below 2^64)
+  // unit rows of a product of at most TX_MAX_GATES gates (the bound is theirs,
+  // so a planned pass never fails here): well inside the digits' bounds
+  // (|G| < 2^62.9 keeps G + bias below 2^64)
   constexpr int64_t LIM = (int64_t(1) << 62) + (int64_t(1) << 42);
   for (int r = 0; r < 16; ++r)
     for (int c = 0; c < 16; ++c) {
@@ -1696,7 +1708,10 @@ void plan_tensor_block(const std::vector<HostOp>& ops, int n, const FxBlock& who
     uint64_t cw = 0;
     for (int j = 0; j < core.G; ++j) cw |= uint64_t(1) << core.order[j];
     std::vector<int> wait, post;
-    for (int i : pending) (op_bits(ops[i]) & ~cw || ops[i].type == OP_SIGN ? wait : core.idx).push_back(i);
+    for (int i : pending) {
+      const bool stays = (op_bits(ops[i]) & ~cw) || ops[i].type == OP_SIGN || core.idx.size() >= TX_MAX_GATES / 2;
+      (stays ? wait : core.idx).push_back(i);
+    }
     uint64_t seen = 0;
     for (int i : seg) {
       const HostOp& op = ops[i];

@@ -34,3 +34,41 @@ def test_entries_of_two_stay_in_fp64(value):
     for make in (lambda v: (np.diag([v, 1.0]), (0,)), lambda v: (np.diag([1.0, 1.0, v, 1.0]), (0, 1))):
         assert [kind for kind, _ in _plan([gate, make(value)])].count(5) == 1
         assert [kind for kind, _ in _plan([gate, make(below)])] == [6]
+
+
+def _window_gates(count, scale):
+    rng = np.random.default_rng(5)
+    return [(_haar(rng, 4) * scale, ([0, 1], [1, 2], [2, 3])[i % 3]) for i in range(count)]
+
+
+@pytest.mark.parametrize("extra", [0, 300])
+def test_long_runs_on_one_window_are_cut(extra):
+    """A gate may be off unitarity by 1e-9, and the integers of a pass leave
+    1 + 2^-20 for its norm: a pass takes at most 256 gates, the diagonals that
+    wait for it included, whatever the length of the run."""
+    diags = [(np.diag(np.exp(1j * np.arange(4) * (i + 1))), (i % 4, (i + 1) % 4)) for i in range(extra)]
+    plan = _plan(diags + _window_gates(3000, 1 + 4e-10))
+    assert max(ops for kind, ops in plan if kind == 6) <= 256
+    assert sum(ops for kind, ops in plan if kind == 6) >= 2500
+
+
+@pytest.mark.gpu
+def test_long_runs_off_unitarity():
+    """3000 gates, each 4e-10 above unit norm, and the result grown by all of
+    them: once refused by the pass after earlier ones had run."""
+    import quantumflow_gb300 as qf
+    n, growth = 11, 4e-10
+    ops = _window_gates(3000, 1 + growth)
+    got = qf.Circuit([qf.Gate(m, qubits=list(q)) for m, q in ops]).run(qf.zero_state(n)).asarray().reshape(-1)
+    psi = np.zeros((2,) * 4, np.clongdouble)
+    psi[0, 0, 0, 0] = 1
+    for m, q in ops:
+        t = np.moveaxis(psi, q, (0, 1)).reshape(4, 4)
+        t = (m.astype(np.clongdouble)[:, :, None] * t[None]).sum(axis=1)
+        psi = np.moveaxis(t.reshape((2,) * 4), (0, 1), q)
+    want = np.zeros(2 ** n, complex)
+    want[:: 2 ** (n - 4)] = psi.reshape(-1)
+    assert abs(np.linalg.norm(want) - (1 + growth) ** 3000) < 1e-9
+    # a pass errs by 2^-55 of its row's largest part and one rounding, at most
+    # 3000 / 32 of them
+    assert np.max(np.abs(got - want)) < 94 * 2.0 ** -52
