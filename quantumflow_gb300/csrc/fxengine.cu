@@ -1214,24 +1214,69 @@ inline Cdd cdd_mul(cplx g, const Cdd& v) {
           dd_add(dd_mul_d(v.im, g.real()), dd_mul_d(v.re, g.imag()))};
 }
 inline Cdd cdd_add(const Cdd& a, const Cdd& b) { return {dd_add(a.re, b.re), dd_add(a.im, b.im)}; }
-// The pass unitary as 2^62 integers.  A gate's entries are rounded to that
-// grid and products are exact in 128 bits, rounded once per gate and entry:
-// k gates err by at most about k 2^-62, below the 2^-59 truncation of every
-// amplitude of the pass.  A product touches only the entries that can be
-// nonzero (rows and columns that agree outside the bits of the gates so far).
-// Three 4x4 gates on a window: 25 -> 10 us of host time a pass, launch included,
-// against double-double products over all entries.
+// The pass unitary, carried to 2^-124 and rounded once, at the end, to the
+// 2^62 integers of the kernel (the products in double-double this replaces
+// were good to 2^-106).  Entries and gates are pairs of integers, (h, l) =
+// (h 2^62 + l) 2^-124: a gate's FP64 entry is such a pair exactly down to
+// 2^-124 (l is 0 from 2^-10 up), and a product takes h h' whole and the upper
+// half of h l' + l h'.  A product touches only the entries that can be nonzero
+// (rows and columns that agree outside the bits of the gates so far).
 using i128 = __int128;
-inline int64_t fixed62(double v) { return std::llround(std::ldexp(v, 62)); }
-inline int64_t round62(i128 v) { return static_cast<int64_t>((v + (i128(1) << 61)) >> 62); }
+struct Fx124 {
+  int64_t h, l;
+};
+inline Fx124 fixed124(double v) {  // |v| < 2
+  if (v == 0.0) return {0, 0};
+  const double s = v * 0x1p62;
+  const int64_t h = std::llround(s);
+  return {h, std::llround((s - static_cast<double>(h)) * 0x1p62)};  // both steps exact
+}
+struct Gate124 {
+  int64_t rh, ih, rl, il;
+  bool low() const { return (rl | il) != 0; }
+  bool zero() const { return (rh | ih | rl | il) == 0; }
+};
+inline Gate124 gate124(cplx v) {
+  const Fx124 r = fixed124(v.real()), i = fixed124(v.imag());
+  return {r.h, i.h, r.l, i.l};
+}
+inline int64_t round62(i128 v) {  // ties away from zero
+  constexpr i128 half = i128(1) << 61;
+  return static_cast<int64_t>(v < 0 ? -((half - v) >> 62) : (half + v) >> 62);
+}
 struct TxUnitary {
-  int64_t re[16][16], im[16][16];
+  struct Entry {
+    int64_t rh, ih, rl, il;  // 0 <= rl, il < 2^62
+  };
+  Entry u[16][16];
   uint32_t used = 0;  // window bits of the gates so far
+  bool low = false;   // any of the l may be nonzero
   void identity(int shift) {
-    std::memset(re, 0, sizeof(re));
-    std::memset(im, 0, sizeof(im));
-    for (int c = 0; c < 16; ++c) re[c][c] = int64_t(1) << (62 - shift);
+    std::memset(u, 0, sizeof(u));
+    for (int c = 0; c < 16; ++c) u[c][c].rh = int64_t(1) << (62 - shift);
     used = 0;
+    low = false;
+  }
+  static i128 whole(int64_t h, int64_t l) { return i128(h) * (i128(1) << 62) + l; }
+  i128 re(int r, int c) const { return whole(u[r][c].rh, u[r][c].rl); }
+  i128 im(int r, int c) const { return whole(u[r][c].ih, u[r][c].il); }
+  static Entry entry(i128 r, i128 i) {
+    constexpr int64_t mask = (int64_t(1) << 62) - 1;
+    return {static_cast<int64_t>(r >> 62), static_cast<int64_t>(i >> 62), static_cast<int64_t>(r) & mask,
+            static_cast<int64_t>(i) & mask};
+  }
+  // (ar, ai) += g e
+  void muladd(const Gate124& g, const Entry& e, i128& ar, i128& ai) const {
+    ar += i128(g.rh) * e.rh - i128(g.ih) * e.ih;
+    ai += i128(g.rh) * e.ih + i128(g.ih) * e.rh;
+    if (low) {
+      ar += (i128(g.rh) * e.rl - i128(g.ih) * e.il) >> 62;
+      ai += (i128(g.rh) * e.il + i128(g.ih) * e.rl) >> 62;
+    }
+    if (g.low()) {
+      ar += (i128(g.rl) * e.rh - i128(g.il) * e.ih) >> 62;
+      ai += (i128(g.rl) * e.ih + i128(g.il) * e.rh) >> 62;
+    }
   }
   // f(r, c) for the entries that can be nonzero
   template <typename F>
@@ -1242,19 +1287,21 @@ struct TxUnitary {
         if (sub == 0) break;
       }
   }
-  void scale_row_entry(int r, int c, int64_t gr, int64_t gi) {
-    const int64_t ur = re[r][c], ui = im[r][c];
-    re[r][c] = round62(i128(gr) * ur - i128(gi) * ui);
-    im[r][c] = round62(i128(gr) * ui + i128(gi) * ur);
+  // row r of the gates so far times g[factor(r)]
+  template <typename F>
+  void scale_rows(const Gate124* g, F factor) {
+    entries([&](int r, int c) {
+      i128 ar = 0, ai = 0;
+      muladd(g[factor(r)], u[r][c], ar, ai);
+      u[r][c] = entry(ar, ai);
+    });
+    low = true;
   }
   // U <- E U, E the gate m on the window bits jp[0..k) (jp[0] the matrix MSB)
   void apply(const CMat& m, int k, const int* jp) {
     const int D = 1 << k;
-    int64_t gr[256], gi[256];
-    for (int e = 0; e < D * D; ++e) {
-      gr[e] = fixed62(m[e].real());
-      gi[e] = fixed62(m[e].imag());
-    }
+    Gate124 g[256];
+    for (int e = 0; e < D * D; ++e) g[e] = gate124(m[e]);
     uint32_t om = 0;
     int spread[16];
     for (int j = 0; j < k; ++j) om |= 1u << jp[j];
@@ -1264,9 +1311,8 @@ struct TxUnitary {
         if ((x >> (k - 1 - j)) & 1) spread[x] |= 1 << jp[j];
     }
     const uint32_t all = used | om;
-    int64_t tr[16][16], ti[16][16];
-    std::memset(tr, 0, sizeof(tr));
-    std::memset(ti, 0, sizeof(ti));
+    Entry t[16][16];
+    std::memset(t, 0, sizeof(t));
     for (int base = 0; base < 16; ++base) {
       if (base & om) continue;
       for (int x = 0; x < D; ++x) {
@@ -1274,29 +1320,26 @@ struct TxUnitary {
         std::memset(ar, 0, sizeof(ar));
         std::memset(ai, 0, sizeof(ai));
         for (int y = 0; y < D; ++y) {
-          const int64_t er = gr[x * D + y], ei = gi[x * D + y];
-          if (er == 0 && ei == 0) continue;
+          const Gate124& e = g[x * D + y];
+          if (e.zero()) continue;
           const int row = base | spread[y];
           for (uint32_t sub = used;; sub = (sub - 1) & used) {
             const int c = static_cast<int>((row & ~used) | sub);
-            const int64_t ur = re[row][c], ui = im[row][c];
-            ar[c] += i128(er) * ur - i128(ei) * ui;
-            ai[c] += i128(er) * ui + i128(ei) * ur;
+            muladd(e, u[row][c], ar[c], ai[c]);
             if (sub == 0) break;
           }
         }
         const int r = base | spread[x];
         for (uint32_t sub = all;; sub = (sub - 1) & all) {
           const int c = static_cast<int>((r & ~all) | sub);
-          tr[r][c] = round62(ar[c]);
-          ti[r][c] = round62(ai[c]);
+          t[r][c] = entry(ar[c], ai[c]);
           if (sub == 0) break;
         }
       }
     }
-    std::memcpy(re, tr, sizeof(re));
-    std::memcpy(im, ti, sizeof(im));
+    std::memcpy(u, t, sizeof(u));
     used = all;
+    low = true;
   }
 };
 
@@ -1377,8 +1420,8 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
     }
     if (op.type == OP_PHASE) {
       if (!matrix) continue;
-      const int64_t gr = fixed62(op.scalar.real()), gi = fixed62(op.scalar.imag());
-      U.entries([&](int r, int c) { U.scale_row_entry(r, c, gr, gi); });
+      const Gate124 g = gate124(op.scalar);
+      U.scale_rows(&g, [](int) { return 0; });
       continue;
     }
     if (op.type == OP_DIAG) {
@@ -1388,15 +1431,12 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
         if (jp[j] < 0) return QF_ERR_NOT_SUPPORTED;
       }
       if (!matrix) continue;
-      int64_t gr[8], gi[8];
-      for (int e = 0; e < (1 << op.k); ++e) {
-        gr[e] = fixed62(op.diag[e].real());
-        gi[e] = fixed62(op.diag[e].imag());
-      }
-      U.entries([&](int r, int c) {
+      Gate124 g[8];
+      for (int e = 0; e < (1 << op.k); ++e) g[e] = gate124(op.diag[e]);
+      U.scale_rows(g, [&](int r) {
         int e = 0;
         for (int j = 0; j < op.k; ++j) e = (e << 1) | ((r >> jp[j]) & 1);
-        U.scale_row_entry(r, c, gr[e], gi[e]);
+        return e;
       });
       continue;
     }
@@ -1414,10 +1454,7 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
     if (mo == 0) {  // inside the window: a diagonal of U
       if (!matrix) continue;
       U.entries([&](int r, int c) {
-        if ((rm >> r) & 1) {
-          U.re[r][c] = -U.re[r][c];
-          U.im[r][c] = -U.im[r][c];
-        }
+        if ((rm >> r) & 1) U.u[r][c] = TxUnitary::entry(-U.re(r, c), -U.im(r, c));
       });
       continue;
     }
@@ -1446,9 +1483,10 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
   constexpr int64_t LIM = (int64_t(1) << 62) + (int64_t(1) << 42);
   for (int r = 0; r < 16; ++r)
     for (int c = 0; c < 16; ++c) {
-      if (std::abs(U.re[r][c]) > LIM || std::abs(U.im[r][c]) > LIM) return QF_ERR_NOT_SUPPORTED;
-      P.g[r][c][0] = U.re[r][c];
-      P.g[r][c][1] = U.im[r][c];
+      const int64_t re = round62(U.re(r, c)), im = round62(U.im(r, c));
+      if (std::abs(re) > LIM || std::abs(im) > LIM) return QF_ERR_NOT_SUPPORTED;
+      P.g[r][c][0] = re;
+      P.g[r][c][1] = im;
     }
   return QF_OK;
 }
