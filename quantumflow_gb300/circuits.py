@@ -28,10 +28,10 @@ class Circuit(Operation):
 
     def __init__(self, elements: Iterable[Operation] = None) -> None:
         self.elements = list(elements) if elements is not None else []
-        self._pack_flat = None  # the gates, qubits and arrays of the last packing
-        self._pack_qubits = None
-        self._pack = None
-        self._pack_narrow = False
+        # the last packing: its gates, qubits, arrays, and whether every gate
+        # is narrow enough for one launch (one attribute: another thread may
+        # pack the same circuit)
+        self._packing = None
 
     def add(self, other: "Circuit") -> "Circuit":
         return Circuit(self.elements + other.elements)
@@ -76,8 +76,9 @@ class Circuit(Operation):
         return self._packed(self.gates(), tuple(qubits))
 
     def _packed(self, flat, qubits):
-        if self._is_packed(flat, qubits):
-            return self._pack
+        held = self._held(flat, qubits)
+        if held is not None:
+            return held[2]
         index = {q: i for i, q in enumerate(qubits)}
         ks, axes, mats = [], [], []
         for g in flat:
@@ -89,15 +90,18 @@ class Circuit(Operation):
         op_k = np.asarray(ks, dtype=np.int32)
         op_axes = np.asarray(axes, dtype=np.int32)
         op_mats = np.ascontiguousarray(np.concatenate(mats) if mats else np.zeros(1))
-        self._pack_flat, self._pack_qubits = flat, qubits
-        self._pack = (op_k, op_axes, op_mats, len(flat))
-        return self._pack
+        arrays = (op_k, op_axes, op_mats, len(flat))
+        self._packing = (flat, qubits, arrays, max(ks, default=0) <= nat.MAX_GATE_QUBITS)
+        return arrays
 
-    def _is_packed(self, flat, qubits) -> bool:
-        """Whether the arrays at hand are those of these very gates (held by
-        the packing, so none of them can have been replaced)."""
-        return (self._pack_flat is not None and self._pack_qubits == qubits
-                and len(flat) == len(self._pack_flat) and all(map(operator.is_, flat, self._pack_flat)))
+    def _held(self, flat, qubits):
+        """The packing at hand if it is of these very gates (it holds them, so
+        none of them can have been replaced), else None."""
+        held = self._packing
+        if (held is not None and held[1] == qubits and len(flat) == len(held[0])
+                and all(map(operator.is_, flat, held[0]))):
+            return held
+        return None
 
     def run(self, ket: State = None, fusion_k: int = None) -> State:
         """Apply the circuit (quantumflow/circuits.py:87-99); default initial
@@ -109,10 +113,10 @@ class Circuit(Operation):
         flat = self.gates()
         qubits = tuple(ket.qubits)
         # (gates packed before, all of them narrow enough, are not looked at again)
-        if not (self._pack_narrow and self._is_packed(flat, qubits)):
-            self._pack_narrow = all(getattr(g, "_is_gate", False) and g.qubit_nb <= nat.MAX_GATE_QUBITS
-                                    for g in flat)
-        if not self._pack_narrow:
+        held = self._held(flat, qubits)
+        narrow = held[3] if held is not None else all(
+            getattr(g, "_is_gate", False) and g.qubit_nb <= nat.MAX_GATE_QUBITS for g in flat)
+        if not narrow:
             # mixed operations: each run of consecutive gates is one fused
             # launch, other operations (and gates wider than the fused
             # engine takes) run on their own in between
@@ -128,7 +132,7 @@ class Circuit(Operation):
             if pending:
                 ket = Circuit(pending).run(ket, fusion_k)
             return ket
-        op_k, op_axes, op_mats, nops = self._packed(flat, qubits)
+        op_k, op_axes, op_mats, nops = held[2] if held is not None else self._packed(flat, qubits)
         src = ket.buffer.compute()
         out = src if (fresh or src is not ket.buffer) else src.empty_like()
         passes = (nat.ctypes.c_int * 1)()
