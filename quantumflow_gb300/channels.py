@@ -235,17 +235,19 @@ class Dephasing(UnitaryMixture):
 
 
 def narrow_superop(elem):
-    """The superoperator of a channel on one or two qubits that evolves as one
-    pass (its class does not override how), else None."""
-    cls = type(elem)
-    if getattr(cls, "evolve", None) not in (Channel.evolve, Kraus.evolve):
+    """The superoperator, its axes in the order of ``elem.qubits``, of a channel
+    on one or two qubits that evolves as one pass (neither its class nor the
+    object itself overrides how), else None."""
+    how = getattr(getattr(elem, "evolve", None), "__func__", None)
+    if how is not Channel.evolve and how is not Kraus.evolve:
         return None
     k = len(elem.qubits)
     if k > 2:
         return None
-    if cls.evolve is Channel.evolve:
-        return elem.tensor.reshape(4 ** k, 4 ** k)
-    return elem.aschannel().tensor.reshape(4 ** k, 4 ** k)
+    chan = elem if how is Channel.evolve else elem.aschannel()
+    if tuple(chan.qubits) != tuple(elem.qubits):  # a class of its own may order them otherwise
+        return None
+    return chan.tensor.reshape(4 ** k, 4 ** k)
 
 
 def join_channels(*channels: Channel) -> Channel:
