@@ -13,6 +13,7 @@ default) or native FP64, or they are held as float-float pairs
 to complex128 only when ``State.tensor`` is read.
 """
 import math
+import threading
 from collections import defaultdict
 from functools import reduce
 from typing import Any, Dict, TextIO, Union
@@ -123,11 +124,50 @@ class Buffer:
 
 # Sampled counts of these sizes (bytes) are read into page-locked memory
 # (from torch's caching host allocator, as State.to_host's): 32 MiB took
-# 0.2 ms, 2.2 ms through pageable memory.  Larger arrays stay pageable, so
-# that results a program keeps do not lock much memory; below, the
-# allocator's bookkeeping costs what the copy saves.
+# 0.2 ms, 2.2 ms through pageable memory.  Below, the allocator's bookkeeping
+# costs what the copy saves.  Larger arrays stay pageable, and so do all once
+# the arrays that the program still holds lock _PINNED_RESULTS bytes.
 _PAGEABLE_COUNTS = 1 << 18
 _PINNED_COUNTS = 1 << 26
+_PINNED_RESULTS = 1 << 29
+
+
+class _PinnedArray:
+    """Page-locked int64 memory in a caller's hands: the base of the numpy
+    array (and so of its views) that ``array`` makes, counted while any of
+    them lives."""
+
+    _held = 0
+    _lock = threading.RLock()  # (__del__ may run inside it)
+
+    def __init__(self, count: int):
+        self._bytes = 0
+        self.tensor = torch.empty(count, dtype=torch.int64, pin_memory=True)
+        self._count(8 * count)
+
+    @classmethod
+    def make(cls, count: int):
+        """Room for ``count`` entries, or None above _PINNED_RESULTS."""
+        with cls._lock:
+            return cls(count) if cls._held + 8 * count <= _PINNED_RESULTS else None
+
+    def _count(self, nbytes: int) -> None:
+        cls = type(self)
+        with cls._lock:
+            self._bytes += nbytes
+            cls._held += nbytes
+
+    def __del__(self):
+        self._count(-self._bytes)
+
+    @property
+    def __array_interface__(self) -> dict:
+        return {"version": 3, "typestr": np.dtype(np.int64).str, "shape": tuple(self.tensor.shape),
+                "data": (self.tensor.data_ptr(), False)}
+
+    def array(self) -> np.ndarray:
+        return np.asarray(self)
+
 
 _IO_STREAMS = {}
 
@@ -310,7 +350,9 @@ class State:
         return probs.reshape([2] * buf.n)
 
     def sample(self, trials: int, seed: int = None) -> np.ndarray:
-        """Multinomial counts over basis states (quantumflow/states.py:121-129)."""
+        """Multinomial counts over basis states (quantumflow/states.py:121-129).
+        Arrays of 256 KiB to 64 MiB sit in page-locked memory, up to 512 MiB in
+        all of those the program still holds; later ones do not."""
         buf = self._buf
         trials = int(trials)
         nbytes = 8 * 2 ** buf.n
@@ -327,12 +369,12 @@ class State:
         nat.call("qf_sample", nat.ptr(buf.data), buf.n, buf.layout, trials,
                  _next_seed(seed), nat.ptr(counts), nat.ptr(ws), nbytes_ws,
                  nat.stream_handle(buf.device))
-        if nbytes < _PAGEABLE_COUNTS or nbytes > _PINNED_COUNTS:
+        host = _PinnedArray.make(counts.numel()) if _PAGEABLE_COUNTS <= nbytes <= _PINNED_COUNTS else None
+        if host is None:
             return counts.cpu().numpy().reshape([2] * buf.n)
-        host = torch.empty(counts.shape, dtype=torch.int64, pin_memory=True)
-        host.copy_(counts, non_blocking=True)
+        host.tensor.copy_(counts, non_blocking=True)
         torch.cuda.current_stream(buf.device).synchronize()
-        return host.numpy().reshape([2] * buf.n)
+        return host.array().reshape([2] * buf.n)
 
     def _draws(self, trials: int, seed) -> np.ndarray:
         """The basis state of each trial (the draws ``sample`` counts)."""
