@@ -558,8 +558,10 @@ __global__ void k_wave_reduce(const int32_t* seg_begin, const WvSeg* segs, int n
 // ------------------------------------------------------------ host plan ----
 struct WvPlanHeader {
   int32_t magic, layout, rbf, rba;
-  // the schedule in passes of one register group: per instance
-  // 1 + p (m - 1) a sweep (a two-group pass stands for the ones it covers)
+  // The first fields keep their places and meaning for readers of the image:
+  // nwaves, nfwd and nadj count the schedule in passes of one register group,
+  // per instance 1 + p (m - 1) a sweep (a two-group pass stands for the ones
+  // it covers).  What runs is counted below.
   int32_t ninst, nwaves, nfwd, nadj, nsegs, nout;
   // the passes that run: waves (launch rounds), one-group and two-group items
   int32_t rounds, ifwd, iadj, ipfwd, ipadj, pad;
@@ -705,6 +707,11 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
     const int64_t per = pairs(n) ? WP_TILES_ADJ : WV_SUBS_PER_BLOCK;
     return (int32_t)(((int64_t(1) << (n - 5 - (pairs(n) ? 2 : 1) * RBa)) + per - 1) / per);
   };
+  // passes of a sweep that takes one group each (the header's counts)
+  auto one_group = [](int n, int p, int RB) {
+    const int m = (n - 5 + RB - 1) / RB;
+    return m == 1 ? p : 1 + p * (m - 1);
+  };
   int64_t st = 0, ct = 0, tb = 0;
   int nw = 0, nfwd1 = 0, nadj1 = 0, nw1 = 0;
   for (int i = 0; i < ninst; ++i) {
@@ -728,19 +735,18 @@ int wave_plan(const qf_batch_instance* hinst, int ninst, int layout, void* host_
     w.tab = tb;
     tb += wv_tab_size(q.p, q.nedges);
     P.inst.push_back(w);
-    wv_fwd_passes(q.n, q.p, RBf, fw[i]);
-    wv_adj_passes(q.n, q.p, RBa, ad[i], sl[i]);
-    nfwd1 += (int)fw[i].size();
-    nadj1 += (int)ad[i].size();
-    nw1 = std::max(nw1, (int)(fw[i].size() + ad[i].size()));
+    const int f1 = one_group(q.n, q.p, RBf), a1 = one_group(q.n, q.p, RBa);
+    nfwd1 += f1;
+    nadj1 += a1;
+    nw1 = std::max(nw1, f1 + a1);
     if (pairs(q.n)) {
-      fw[i].clear();
-      ad[i].clear();
-      sl[i].clear();
       pf[i] = pair_fwd_passes(q.n, q.p, RBf);
       pa[i] = pair_adj_passes(q.n, q.p, RBa);
       for (const PairPass& a : pa[i])
         sl[i].push_back({q.p + a.layerA, a.cost ? a.layerA : -1, a.init ? 2 * q.p : -1, a.hasB ? q.p + a.layerB : -1});
+    } else {
+      wv_fwd_passes(q.n, q.p, RBf, fw[i]);
+      wv_adj_passes(q.n, q.p, RBa, ad[i], sl[i]);
     }
     nw = std::max(nw, (int)(fw[i].size() + ad[i].size() + pf[i].size() + pa[i].size()));
   }
