@@ -714,6 +714,12 @@ constexpr int FX_G_MAX = 4;
 // 1 + 2 FX_UNIT_TOL (4x4), and 256 of them stay below 1 + 2^-20, the bound the
 // pass's digits are laid out for.
 constexpr int TX_MAX_GATES = 256;
+// Most diagonals that wait for a later window before they run in passes of
+// their own: every block looks through those that wait (8000 gates, diagonals
+// on one half of 16 qubits and dense gates on the other: planning 29 ms without
+// a limit, growing with the square; 8 with it).  A Fourier transform of 32
+// qubits has about 250 waiting.
+constexpr size_t TX_MAX_WAITING = 256;
 static_assert(TX_MAX_GATES * 2 * FX_UNIT_TOL < 0x1p-20, "norm of a window");
 
 // Greedy passes: element-wise ops join the current pass; a dense op joins
@@ -1863,7 +1869,8 @@ std::vector<FxBlock> fx_plan_final(std::vector<HostOp>& ops, int n, int& fusion_
     for (int i : B.idx) phases = phases && (phase_op(ops[i]) || ops[i].type == OP_DENSE1 || ops[i].type == OP_DENSE2);
     if (phases && B.G == 0) {
       pending.insert(pending.end(), B.idx.begin(), B.idx.end());
-      if (fusion_k == 1) emit_phases(ops, pending, everything, out);
+      // (a phase pass takes 48 signs and looks through all that wait)
+      if (fusion_k == 1 || pending.size() > 16 * TX_MAX_WAITING) emit_phases(ops, pending, everything, out);
       continue;
     }
     if (!phases) {  // a three-qubit diagonal: the interpreted kernels
@@ -1880,6 +1887,7 @@ std::vector<FxBlock> fx_plan_final(std::vector<HostOp>& ops, int n, int& fusion_
       }
       continue;
     }
+    if (pending.size() > TX_MAX_WAITING) emit_phases(ops, pending, everything, out);
     plan_tensor_block(ops, n, B, pending, out, fusion_k);
   }
   emit_phases(ops, pending, everything, out);

@@ -72,3 +72,18 @@ def test_long_runs_off_unitarity():
     # a pass errs by 2^-55 of its row's largest part and one rounding, at most
     # 3000 / 32 of them
     assert np.max(np.abs(got - want)) < 94 * 2.0 ** -52
+
+
+def test_waiting_diagonals_are_bounded():
+    """Diagonals that no later gate touches do not pile up while a long circuit
+    is planned: a phase pass of them every few hundred."""
+    rng = np.random.default_rng(4)
+    ops = []
+    for _ in range(6000):
+        a, b = (int(x) for x in rng.choice(6, 2, replace=False))
+        ops.append((np.diag(np.exp(1j * rng.uniform(0, 6, 4))), (a, b)) if rng.random() < 0.5
+                   else (_haar(rng, 4), (6 + a, 6 + b)))
+    plan = _plan(ops)
+    waiting = [count for kind, count in plan if kind == 0]
+    assert max(waiting) <= 256 + 128 and len(waiting) >= 4
+    assert sum(count for kind, count in plan if kind in (0, 6)) > 4000
