@@ -1516,7 +1516,16 @@ uint64_t op_bits(const HostOp& op) {
 // window of at most four bits that has a bit of every two-qubit diagonal it
 // takes (the most frequent bits first).  Ops of the list that a pass can
 // take along go with it; the rest stay in `list`.
-void emit_phases(const std::vector<HostOp>& ops, std::vector<int>& list, uint64_t must, std::vector<FxBlock>& out) {
+// A window gets at least two bits while there are any that no two-qubit
+// diagonal touches: a thread with one or two amplitudes has too few loads in
+// flight.  One CZ, n = 24: 163 us without window bits, 116 with two (the
+// element-wise group pass 128); one RZ 206, 156 (170); n = 28 3739, 2587
+// (2643).  On a bit that a two-qubit diagonal of the pass shares, the phase
+// of the pair would cost a product an amplitude instead (six CPHASEs on one
+// qubit, n = 24: 132 -> 159).
+void emit_phases(const std::vector<HostOp>& ops, int n, std::vector<int>& list, uint64_t must,
+                 std::vector<FxBlock>& out) {
+  constexpr int MIN_WINDOW = 2;
   auto two = [&](int i) { return ops[i].type == OP_DIAG && ops[i].k == 2; };
   for (;;) {
     bool any = false;
@@ -1544,6 +1553,19 @@ void emit_phases(const std::vector<HostOp>& ops, std::vector<int>& list, uint64_
       if (left) break;
       if (pass == 0) continue;
     }
+    uint64_t taken = win;
+    for (int i : list)
+      if (two(i)) taken |= op_bits(ops[i]);
+    auto widen = [&](int b) {
+      if (B.G >= MIN_WINDOW || ((taken >> b) & 1)) return;
+      B.order[B.G++] = b;
+      taken |= uint64_t(1) << b;
+      win |= uint64_t(1) << b;
+    };
+    for (int i : list)  // bits of ops first: their tables then have one factor less
+      if (!two(i))
+        for (int j = 0; j < ops[i].k && ops[i].type != OP_PHASE; ++j) widen(ops[i].gb[j]);
+    for (int b = n - 1; b >= 0; --b) widen(b);
     std::vector<int> rest;
     int nsign = 0;
     for (int i : list) {
@@ -1777,7 +1799,7 @@ void plan_tensor_block(const std::vector<HostOp>& ops, int n, const FxBlock& who
       }
     }
     // core.idx holds ops in circuit order behind the absorbed ones
-    emit_phases(ops, wait, dense, out);
+    emit_phases(ops, n, wait, dense, out);
     pending.swap(wait);
     pending.insert(pending.end(), post.begin(), post.end());
     if (core.idx.empty()) continue;
@@ -1857,7 +1879,7 @@ std::vector<FxBlock> fx_plan_final(std::vector<HostOp>& ops, int n, int& fusion_
   const uint64_t everything = ~uint64_t(0);
   for (FxBlock& B : blocks) {
     if (B.native || B.wide || B.shape == FXB_SWAP) {
-      emit_phases(ops, pending, everything, out);
+      emit_phases(ops, n, pending, everything, out);
       if (B.wide) {  // a 3- or 4-qubit gate: alone on the tensor cores, else native FP64
         if (tx_prepare(n, ops, B, tp, false) == QF_OK) B.shape = FXB_TENSOR;
         else B.native = true;
@@ -1870,11 +1892,11 @@ std::vector<FxBlock> fx_plan_final(std::vector<HostOp>& ops, int n, int& fusion_
     if (phases && B.G == 0) {
       pending.insert(pending.end(), B.idx.begin(), B.idx.end());
       // (a phase pass takes 48 signs and looks through all that wait)
-      if (fusion_k == 1 || pending.size() > 16 * TX_MAX_WAITING) emit_phases(ops, pending, everything, out);
+      if (fusion_k == 1 || pending.size() > 16 * TX_MAX_WAITING) emit_phases(ops, n, pending, everything, out);
       continue;
     }
     if (!phases) {  // a three-qubit diagonal: the interpreted kernels
-      emit_phases(ops, pending, everything, out);
+      emit_phases(ops, n, pending, everything, out);
       std::vector<FxBlock> parts = fx_blocks(ops, B.idx, fusion_k, false);
       for (FxBlock& part : parts) {
         if (part.G > 0 && tx_prepare(n, ops, part, tp, false) == QF_OK) {
@@ -1887,10 +1909,10 @@ std::vector<FxBlock> fx_plan_final(std::vector<HostOp>& ops, int n, int& fusion_
       }
       continue;
     }
-    if (pending.size() > TX_MAX_WAITING) emit_phases(ops, pending, everything, out);
+    if (pending.size() > TX_MAX_WAITING) emit_phases(ops, n, pending, everything, out);
     plan_tensor_block(ops, n, B, pending, out, fusion_k);
   }
-  emit_phases(ops, pending, everything, out);
+  emit_phases(ops, n, pending, everything, out);
   if (fusion_k > 1) absorb_channels(ops, n, out);
   return out;
 }
