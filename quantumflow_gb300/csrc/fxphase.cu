@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(FXP_THREADS, CTAS) k_fxphase(const __grid_cons
     // phases of the low two window bits, then the others outermost
     constexpr int GI = G < 2 ? G : 2, NI = 1 << GI, NO = 1 << (G - GI);
     Phase inner[NI];
-    if constexpr (GI >= 1) inner[1] = fn[0];
+    inner[1] = fn[0];
     if constexpr (GI >= 2) {
       inner[2] = fn[1];
       inner[3] = fxp_mul(fn[0], fn[1]);
@@ -188,11 +188,16 @@ __global__ void __launch_bounds__(FXP_THREADS, CTAS) k_fxphase(const __grid_cons
   }
 }
 
+// tables beyond the thread's own, and the bytes of all of them
+constexpr int fxp_chunks(int n, int G) { return n - G <= FXP_LOW ? 0 : (n - G - 1) / FXP_LOW; }
+constexpr int fxp_smem(int n, int G) { return (1 + fxp_chunks(n, G)) * (G + 1) * (16 << FXP_LOW); }
+constexpr int SM_SMEM = 228 << 10;  // of an SM, 1 KiB of it reserved per CTA
+
 template <int G, typename IT, int CTAS>
 int phase_launch_t(const FxPhaseParams& P, cudaStream_t stream) {
   const int hbits = P.n - G - FXP_LOW;
-  const int nch = hbits <= 0 ? 0 : (hbits + FXP_LOW - 1) / FXP_LOW;
-  const size_t smem = (size_t)(1 + nch) * (G + 1) * (16 << FXP_LOW);
+  const int nch = fxp_chunks(P.n, G);
+  const size_t smem = (size_t)fxp_smem(P.n, G);
   static std::atomic<int> attr_set[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
@@ -271,16 +276,30 @@ __global__ void __launch_bounds__(FXSW_THREADS) k_fxswap(const __grid_constant__
 // Three CTAs an SM from 2^11 tiles of 256 threads (five rounds of them) on,
 // where they hide more of each other's latency: QFT, n = 24 1595 -> 1560 us,
 // n = 26 6731 -> 6530; below, the last round is emptier than with two: n = 21
-// 249 with two, 265 with three.
+// 249 with two, 265 with three.  Only while the tables of three fit an SM
+// (four window bits: up to n = 28): four CPHASEs, n = 29, 5223 us with a grid
+// for three of which two fit, 4000 with two.
+constexpr int phase_ctas(int n, int G) {
+  return n - G - FXP_LOW >= 11 && 3 * (fxp_smem(n, G) + 1024) <= SM_SMEM ? 3 : 2;
+}
+constexpr bool phase_ctas_fit() {
+  for (int n = 11; n <= QF_MAX_QUBITS; ++n)
+    for (int G = 1; G <= 4; ++G)
+      if (phase_ctas(n, G) * (fxp_smem(n, G) + 1024) > SM_SMEM) return false;
+  return true;
+}
+static_assert(phase_ctas_fit(), "a grid of CTAs that are all resident");
+
 template <int G>
 static int phase_launch(const FxPhaseParams& P, cudaStream_t stream) {
-  if (P.n > 31) return phase_launch_t<G, int64_t, 3>(P, stream);
-  return P.n - G - FXP_LOW >= 11 ? phase_launch_t<G, uint32_t, 3>(P, stream) : phase_launch_t<G, uint32_t, 2>(P, stream);
+  const bool three = phase_ctas(P.n, G) == 3;
+  if (P.n > 31)
+    return three ? phase_launch_t<G, int64_t, 3>(P, stream) : phase_launch_t<G, int64_t, 2>(P, stream);
+  return three ? phase_launch_t<G, uint32_t, 3>(P, stream) : phase_launch_t<G, uint32_t, 2>(P, stream);
 }
 
 int fx_phase_launch(const FxPhaseParams& P, cudaStream_t stream) {
   switch (P.G) {
-    case 0: return phase_launch<0>(P, stream);
     case 1: return phase_launch<1>(P, stream);
     case 2: return phase_launch<2>(P, stream);
     case 3: return phase_launch<3>(P, stream);
