@@ -323,7 +323,6 @@ QF_D double2 cmul_v(const Coef& c, double2 a) {
   return make_double2(fma(ur, a.x, -ui * a.y), fma(ur, a.y, ui * a.x));
 }
 // by a coefficient whose imaginary part is 0: two FP64 operations, not four
-QF_D float2 cmul_real(const Coef& c, float2 a) { return make_float2(c.f[0] * a.x, c.f[0] * a.y); }
 QF_D double2 cmul_real(const Coef& c, double2 a) { return make_double2(c.d[0] * a.x, c.d[0] * a.y); }
 QF_D float4 cmul_v(const Coef& c, float4 a) {
   float4 r;
