@@ -130,6 +130,11 @@ class Buffer:
 _PAGEABLE_COUNTS = 1 << 18
 _PINNED_COUNTS = 1 << 26
 _PINNED_RESULTS = 1 << 29
+# Outcomes per trial from which the draws are listed and counted on the host.
+# Counting takes 9 to 12 ns a trial there, the copy of all counts 0.24 ns an
+# outcome: n = 24, 1000 trials 2.5 ms against 6.6, 10^6 trials 11.9 against
+# 6.6; n = 26, 10^6 trials 19.0 against 21.3.
+_DRAW_RATIO = 64
 
 
 class _PinnedArray:
@@ -356,7 +361,7 @@ class State:
         buf = self._buf
         trials = int(trials)
         nbytes = 8 * 2 ** buf.n
-        if nbytes > _PINNED_COUNTS and 0 <= 8 * trials <= 2 ** buf.n:
+        if nbytes > _PINNED_COUNTS and 0 <= _DRAW_RATIO * trials <= 2 ** buf.n:
             # few trials of a large state: read back the drawn states and
             # count them here (torch zeroes the array on all cores; numpy's
             # lazy zero pages would cost one page fault per outcome)

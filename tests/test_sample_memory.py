@@ -58,3 +58,37 @@ def test_results_a_program_keeps_do_not_lock_memory_without_end(monkeypatch):
     del kept[0], counts
     gc.collect()
     assert torch.from_numpy(ket.sample(10, seed=9)).is_pinned()
+
+
+@pytest.mark.gpu
+def test_each_way_to_the_counts(monkeypatch):
+    """Ordinary, page-locked and listed read-backs of one seed, with the sizes
+    brought down; draws are listed for at most one trial in 64 outcomes."""
+    import quantumflow_gb300 as qf
+    from quantumflow_gb300 import states
+    n = 12
+    ket = qf.random_state(n)
+    listed = []
+    draws = states.State._draws
+    monkeypatch.setattr(states.State, "_draws", lambda self, trials, seed: listed.append(trials) or
+                        draws(self, trials, seed))
+    for pageable, pinned in ((1 << 30, 1 << 31), (1 << 10, 1 << 31), (1 << 10, 1 << 11)):
+        monkeypatch.setattr(states, "_PAGEABLE_COUNTS", pageable)
+        monkeypatch.setattr(states, "_PINNED_COUNTS", pinned)
+        for trials in (0, 1, 2 ** n // 64, 2 ** n // 64 + 1, 2 ** n // 8, 2 ** n):
+            listed.clear()
+            counts = ket.sample(trials, seed=77)
+            assert bool(listed) == (pinned == 1 << 11 and 64 * trials <= 2 ** n)
+            assert counts.shape == (2,) * n and counts.dtype == np.int64
+            want = np.bincount(draws(ket, trials, 77), minlength=2 ** n)
+            assert np.array_equal(counts.reshape(-1), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("trials", [1, 1000, 2 ** 24 // 64, 2 ** 24 // 64 + 1])
+def test_counts_of_a_large_state(trials):
+    """n = 24, on both sides of the rule, unpatched."""
+    import quantumflow_gb300 as qf
+    ket = qf.random_state(24)
+    counts = ket.sample(trials, seed=5)
+    assert np.array_equal(counts.reshape(-1), np.bincount(ket._draws(trials, seed=5), minlength=2 ** 24))
