@@ -100,11 +100,11 @@ __global__ void __launch_bounds__(256) k_dense1(const typename Types<LAY>::E* in
       c[0] = in[j0];
       c[1] = in[j0 | bit];
     }
-    out[i0] = cdot<2>(&u.c[0], a);
-    out[i0 | bit] = cdot<2>(&u.c[2], a);
+    out[i0] = cdot_direct<2>(&u.c[0], a);
+    out[i0 | bit] = cdot_direct<2>(&u.c[2], a);
     if (has2) {
-      out[j0] = cdot<2>(&u.c[0], c);
-      out[j0 | bit] = cdot<2>(&u.c[2], c);
+      out[j0] = cdot_direct<2>(&u.c[0], c);
+      out[j0 | bit] = cdot_direct<2>(&u.c[2], c);
     }
   }
 }
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256) k_dense2(const typename Types<LAY>::E* in
       }
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r) out[idx[r]] = cdot<4>(&u.c[4 * r], a);
+    for (int r = 0; r < 4; ++r) out[idx[r]] = cdot_direct<4>(&u.c[4 * r], a);
   }
 }
 

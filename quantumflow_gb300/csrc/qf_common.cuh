@@ -95,28 +95,36 @@ QF_D float2 cdot(const Coef* u, const float2* a) {
 }
 
 // v != 0.0 as an integer test: a floating-point compare is one of the ~2
-// lanes per clock and SM of the FP64 pipe, which bounds these kernels.
-// k_dense2 with 6 real entries, n = 22: 193 -> 131 us.
+// lanes per clock and SM of the FP64 pipe.
 QF_D bool nonzero(double v) {
   return ((static_cast<uint32_t>(__double2hiint(v)) << 1) | static_cast<uint32_t>(__double2loint(v))) != 0u;
 }
-template <int J>
+template <int J, bool DIRECT = false>
 QF_D double2 cdot(const Coef* u, const double2* a) {
   double re = 0.0, im = 0.0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     const double ur = u[j].d[0], ui = u[j].d[1];
-    if (nonzero(ur)) {
+    if (DIRECT ? nonzero(ur) : ur != 0.0) {
       re = fma(ur, a[j].x, re);
       im = fma(ur, a[j].y, im);
     }
-    if (nonzero(ui)) {
+    if (DIRECT ? nonzero(ui) : ui != 0.0) {
       re = fma(-ui, a[j].y, re);
       im = fma(ui, a[j].x, im);
     }
   }
   return make_double2(re, im);
 }
+// cdot for the one-gate sweeps, which the FP64 pipe bounds (k_dense2 with 6
+// real entries, n = 22: 193 -> 131 us with the integer tests).  The kernels
+// that run many ops from shared memory keep the compares: with the tests in
+// every branch their register count doubled (k_tile in complex128 80 -> 158)
+// and a five-qubit gate on 10 qubits took 486 us instead of 291.
+template <int J>
+QF_D float2 cdot_direct(const Coef* u, const float2* a) { return cdot<J>(u, a); }
+template <int J>
+QF_D double2 cdot_direct(const Coef* u, const double2* a) { return cdot<J, true>(u, a); }
 
 // Error-free product terms: p = ah*bh rounded, c = its rounding error plus
 // the ah*bl and al*bh cross terms (the al*bl term, 2^-48 relative, is
@@ -258,6 +266,8 @@ QF_D double2 cmul_add2(double2 u0, double2 a0, double2 u1, double2 a1) {
 QF_D float4 cmul_add2(float4 u0, float4 a0, float4 u1, float4 a1) { return ff_cmac2(u0, a0, u1, a1); }
 
 // single complex multiply by a uniform coefficient
+template <int J>
+QF_D float4 cdot_direct(const Coef* u, const float4* a) { return cdot<J>(u, a); }
 QF_D float2 cmul(const Coef& u, float2 a) { return cdot<1>(&u, &a); }
 QF_D double2 cmul(const Coef& u, double2 a) { return cdot<1>(&u, &a); }
 QF_D float4 cmul(const Coef& u, float4 a) { return cdot<1>(&u, &a); }
