@@ -579,7 +579,7 @@ static int launch_adjw(AdjWParams& P, int grid, cudaStream_t stream) {
   }
   const size_t necoef = (size_t)(2 * P.ndiag + P.ncut);
   const size_t smem = ((necoef * sizeof(Coef) + 127) & ~size_t(127)) + adjw_ring_bytes<LAY, RB>();
-  return pdl_launch(k_adjw<LAY, RB>, grid, 256, smem, stream, P);
+  return pdl_launch_fp32<LAY>(k_adjw<LAY, RB>, grid, 256, smem, stream, P);
 }
 
 // Warp-tile adjoint sweep (k_adjw); psi holds the forward state.  Per layer
@@ -692,7 +692,7 @@ static int launch_adj(AdjParams& P, int grid, cudaStream_t stream) {
     if (rc) return rc;
     attr[dev].store(true);
   }
-  return pdl_launch(k_adj<LAY>, grid, 256, smem, stream, P);
+  return pdl_launch_fp32<LAY>(k_adj<LAY>, grid, 256, smem, stream, P);
 }
 
 // out[0..p) = d<C>/d gamma, out[p..2p) = d<C>/d beta, out[2p] = <C>.

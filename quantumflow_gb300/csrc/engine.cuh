@@ -380,5 +380,19 @@ int pdl_launch(void (*kernel)(P...), int64_t grid, int threads, size_t smem, cud
   cfg.numAttrs = 1;
   return check_cuda(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
+// ... except in native FP64: a pass that does not fill the chip leaves room
+// beside its CTAs, where the next pass's wait; they then share SMs (and their
+// FP64 pipe, the bound of these kernels) while others idle.  QAOA state, p = 4,
+// n = 18: 259 us launched in turn, 557 overlapped; gradient, n = 17: 940, 1368.
+template <int LAY, typename... P, typename... A>
+int pdl_launch_fp32(void (*kernel)(P...), int64_t grid, int threads, size_t smem, cudaStream_t stream,
+                    const A&... args) {
+  if constexpr (LAY == C128) {
+    kernel<<<(unsigned)grid, threads, smem, stream>>>(args...);
+    return check_cuda(cudaGetLastError());
+  } else {
+    return pdl_launch(kernel, grid, threads, smem, stream, args...);
+  }
+}
 
 }  // namespace qf

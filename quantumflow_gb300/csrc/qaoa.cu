@@ -209,7 +209,7 @@ static int launch_qw(QaoaWParams& P, cudaStream_t stream) {
   int64_t grid = (nsub + 7) / 8;
   const int64_t cap = (int64_t)device_sm_count() * 4;
   if (grid > cap) grid = cap;
-  return pdl_launch(k_qaoaw<LAY, RB>, grid, 256, smem, stream, P);
+  return pdl_launch_fp32<LAY>(k_qaoaw<LAY, RB>, grid, 256, smem, stream, P);
 }
 
 static int qaoa_state_warp(void* psi, int n, int layout, const uint16_t* cuts, int nedges, int p,
