@@ -241,11 +241,12 @@ def narrow_superop(elem):
     how = getattr(getattr(elem, "evolve", None), "__func__", None)
     if how is not Channel.evolve and how is not Kraus.evolve:
         return None
-    k = len(elem.qubits)
+    qubits = tuple(elem.qubits)
+    k = len(qubits)
     if k > 2:
         return None
     chan = elem if how is Channel.evolve else elem.aschannel()
-    if tuple(chan.qubits) != tuple(elem.qubits):  # a class of its own may order them otherwise
+    if chan.qubits != qubits:  # a class of its own may order them otherwise
         return None
     return chan.tensor.reshape(4 ** k, 4 ** k)
 

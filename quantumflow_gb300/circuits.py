@@ -151,23 +151,29 @@ class Circuit(Operation):
         from .densities import evolve_gates
         if rho is None:
             rho = zero_state(self.qubits).asdensity()
+        elems = self.gates()
         # channels join the launch where the planner takes them into a gate
-        # pass or runs them in FP64 (fixed point) or a merged pass costs the same
-        join = rho.dtype == "complex64" or config.C128_ARITHMETIC == "fx"
-        pending = []
-        for elem in self.gates():
+        # pass or runs them in FP64 (fixed point) or a merged pass costs the
+        # same; one that is alone costs less through its own entry point
+        join = len(elems) > 1 and (rho.dtype == "complex64" or config.C128_ARITHMETIC == "fx")
+        ops, alone = [], None  # alone: the channel, if `ops` is just one
+        for elem in elems:
             if getattr(elem, "_is_gate", False):
-                pending.append(elem)
+                ops.append(elem)
+                alone = None
                 continue
             superop = narrow_superop(elem) if join else None
             if superop is not None:
-                pending.append((superop, elem.qubits))
+                alone = None if ops else elem
+                ops.append((superop, elem.qubits))
                 continue
-            if pending:
-                rho = evolve_gates(rho, pending)
-                pending = []
+            if ops:
+                rho = alone.evolve(rho) if alone is not None else evolve_gates(rho, ops)
+                ops, alone = [], None
             rho = elem.evolve(rho)
-        return evolve_gates(rho, pending) if pending else rho
+        if alone is not None:
+            return alone.evolve(rho)
+        return evolve_gates(rho, ops) if ops else rho
 
     def aschannel(self):
         """Composite superoperator of the elements, in order."""

@@ -29,6 +29,30 @@ def test_a_channel_in_its_own_order_keeps_its_pass():
     assert narrow_superop(damp) is None
 
 
+def test_a_channel_alone_runs_by_itself(monkeypatch):
+    """Which launches a circuit of gates and channels makes (recorded, not
+    made): one for every run of two or more, a lone channel through its own
+    entry point."""
+    import quantumflow_gb300 as qf
+    from quantumflow_gb300 import channels, densities
+    seen = []
+
+    class Rho:
+        dtype = "complex128"
+
+    monkeypatch.setattr(densities, "evolve_gates", lambda rho, ops: seen.append(len(ops)) or rho)
+    monkeypatch.setattr(channels, "evolve_superop", lambda rho, *a: seen.append("alone") or rho)
+    damp = lambda q: qf.Damping(0.1, q)
+    wide = qf.join_channels(*(damp(q).aschannel() for q in range(3)))  # three qubits: always by itself
+    for elems, want in (([damp(0)], ["alone"]), ([damp(0), damp(1)], [2]), ([qf.X(0), damp(0)], [2]),
+                        ([damp(0), qf.X(0)], [2]), ([qf.X(0)], [1]),
+                        ([damp(0), wide, damp(1)], ["alone"] * 3), ([qf.X(0), wide, damp(1), damp(2)], [1, "alone", 2]),
+                        ([], [])):
+        seen.clear()
+        qf.Circuit(elems).evolve(Rho())
+        assert seen == want
+
+
 @pytest.mark.gpu
 def test_evolution_with_a_channel_in_its_own_order():
     import quantumflow_gb300 as qf
