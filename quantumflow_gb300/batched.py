@@ -75,6 +75,7 @@ class QAOABatch:
         # offsets in the caller's (input) order; launch order is largest first
         self.angle_offset = np.concatenate([[0], np.cumsum(2 * self.ps)[:-1]]).astype(np.int64)
         self.out_offset = np.concatenate([[0], np.cumsum(2 * self.ps + 1)[:-1]]).astype(np.int64)
+        self._energy_index = self.out_offset + 2 * self.ps
         self.edge_offset = np.concatenate([[0], np.cumsum(self.nedges)[:-1]]).astype(np.int64)
         edges = np.concatenate(edges_all) if edges_all else np.zeros((0, 2), np.uint8)
         self.d_edges = torch.from_numpy(np.ascontiguousarray(edges).reshape(-1)).to(self.device)
@@ -208,7 +209,7 @@ class QAOABatch:
             dgs.append(o[off:off + p].copy())
             dbs.append(o[off + p:off + 2 * p].copy())
             off += 2 * p + 1
-        return o[self.out_offset + 2 * self.ps], dbs, dgs
+        return o[self._energy_index], dbs, dgs
 
     # ------------------------------------------------------------ Adam -----
     def optimizer_reset(self, maxcut=None, target=None):
