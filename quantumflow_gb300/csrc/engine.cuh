@@ -342,8 +342,7 @@ struct TxParams {
   int32_t n, nin, nout;
   int32_t shift;                    // U is stored scaled by 2^-shift (0 for a unitary)
   int32_t sbits[4];                 // window bits, ascending
-  int64_t off[16];                  // global offset of window index c
-  int64_t boff[16];                 // the same in bytes
+  int64_t boff[16];                 // global offset of window index c, in bytes
   int64_t g[16][16][2];             // U as round(entry * 2^(62 - shift)): [out c][in c][re, im]
   uint64_t in_mout[TX_MAX_SIGNS];   // input-side sign ops: their bits outside the window
   uint64_t out_mout[TX_MAX_SIGNS];  // output-side sign ops

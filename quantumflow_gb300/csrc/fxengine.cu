@@ -1409,7 +1409,6 @@ int tx_prepare(int n, const std::vector<HostOp>& ops, const FxBlock& B, TxParams
     int64_t o = 0;
     for (int j = 0; j < 4; ++j)
       if ((c >> j) & 1) o |= int64_t(1) << wb[j];
-    P.off[c] = o;
     P.boff[c] = 16 * o;
   }
   double norm2 = 1.0;
@@ -1802,11 +1801,9 @@ void plan_tensor_block(const std::vector<HostOp>& ops, int n, const FxBlock& who
       const bool stays = (op_bits(ops[i]) & ~cw) || ops[i].type == OP_SIGN || core.idx.size() >= TX_MAX_GATES / 2;
       (stays ? wait : core.idx).push_back(i);
     }
-    uint64_t seen = 0;
     for (int i : seg) {
       const HostOp& op = ops[i];
       if (is_dense(i)) {
-        seen |= op_bits(op);
         core.idx.push_back(i);
       } else if (op.type == OP_DIAG && (op_bits(op) & ~cw)) {
         // a later dense gate on its bits: it has none before (the segment

@@ -215,8 +215,7 @@ __global__ void __launch_bounds__(QTile<T, RB>::NT, T >= 12 ? 1 : 2) k_qtile(con
   __syncthreads();
   // so far only parameters were read: this may have run while the previous
   // pass drained (programmatic dependent launch)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
   uint32_t tile = blockIdx.x;
   fetch(tile);
   for (; tile < ntiles; tile += gridDim.x) {
@@ -359,17 +358,7 @@ int launch_t(QTileParams& P, cudaStream_t stream) {
         P.off1[r] |= 1u << P.tb[j];
       }
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid_of<T>(P.n));
-  cfg.blockDim = dim3(Q::NT);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute la[1];
-  la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  la[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = la;
-  cfg.numAttrs = 1;
-  return check_cuda(cudaLaunchKernelEx(&cfg, k_qtile<T, RB, ADJ>, P));
+  return pdl_launch(k_qtile<T, RB, ADJ>, grid_of<T>(P.n), Q::NT, smem, stream, P);
 }
 template <bool ADJ>
 int launch(QTileParams& P, int T, cudaStream_t stream) {

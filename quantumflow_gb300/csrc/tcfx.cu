@@ -628,8 +628,7 @@ __global__ void __launch_bounds__(TxShape<AP>::THREADS, 1) k_txpipe(const __grid
   // The prologue above reads only parameters, so it may run while the
   // previous pass of the stream drains (programmatic dependent launch);
   // nothing of the state is touched before that pass has finished.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
   const uint32_t tmem = tmem_slot;
   const int64_t ntiles = (int64_t(1) << (P.n - 4)) / TX_ROWS;
   if (warp < CW) {
@@ -641,7 +640,7 @@ __global__ void __launch_bounds__(TxShape<AP>::THREADS, 1) k_txpipe(const __grid
     const double2* __restrict__ in = static_cast<const double2*>(P.in);
     const int irow = AP == 8 ? warp * 16 + (lane & 7) + ((lane >> 4) << 3) : warp * 8 + (lane & 7);
     const int q = AP == 8 ? (lane >> 3) & 1 : lane >> 3;
-    const int64_t grow = tx_spread(P, irow) | P.off[AP * q];  // this group within its tile
+    const int64_t grow = tx_spread(P, irow) | (P.boff[AP * q] >> 4);  // this group within its tile
     const int64_t step = gridDim.x;
     double2 x[AP];
     int64_t tile = blockIdx.x;
@@ -702,7 +701,7 @@ __global__ void __launch_bounds__(TxShape<AP>::THREADS, 1) k_txpipe(const __grid
     double2* out = static_cast<double2*>(P.out);
     const int ew = warp - CW;
     const int orow = 32 * (ew & 3) + lane, oh = ew >> 2;
-    const int64_t hrow = tx_spread(P, orow) | (oh ? P.off[8] : 0);
+    const int64_t hrow = tx_spread(P, orow) | (oh ? P.boff[8] >> 4 : 0);
     const uint32_t lane_addr = static_cast<uint32_t>(32 * (ew & 3)) << 16;
     int64_t tile = blockIdx.x;
     for (int it = 0; tile < ntiles; tile += gridDim.x, ++it) {
@@ -734,17 +733,7 @@ int tx_launch_ap(const TxParams& P, cudaStream_t stream) {
   const int64_t ntiles = (int64_t(1) << (P.n - 4)) / TX_ROWS;
   int64_t grid = device_sm_count();
   if (grid > ntiles) grid = ntiles;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(TxShape<AP>::THREADS);
-  cfg.dynamicSmemBytes = TP_SMEM;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return check_cuda(cudaLaunchKernelEx(&cfg, k_txpipe<AP>, P));
+  return pdl_launch(k_txpipe<AP>, grid, TxShape<AP>::THREADS, TP_SMEM, stream, P);
 }
 
 }  // namespace
