@@ -20,8 +20,8 @@
 // Arithmetic: an amplitude's two parts share one exponent (57-bit integers,
 // fx.cuh), phases are 2^58 integers multiplied with 2^-57 relative error, and
 // each part is rounded to FP64 once by the exactly rounding convert.
-// Bound: about 220 instructions an amplitude (n = 24: issue 58%, integer ALU
-// 60%), then HBM (32 bytes an amplitude).  QFT, n = 23: 70 us a pass (0.27 GB
+// Bound: 160 to 220 instructions an amplitude (n = 24: issue 50 to 58%, integer
+// ALU 58 to 60%), then HBM (32 bytes an amplitude).  QFT, n = 23: 70 us a pass (0.27 GB
 // moved; 40 us at the copy rate); the interpreted group passes took 950 to
 // 1570 us.
 #include <atomic>

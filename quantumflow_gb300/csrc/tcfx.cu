@@ -6,7 +6,8 @@
 // applied gate by gate (quantumflow/circuits.py:87-99).  A pass applies a
 // run of unitary gates whose dense qubits lie in a window of four bits,
 // with CZ-like sign ops around them (or one unitary gate on 3 or 4
-// qubits): the host multiplies them into one 16x16 unitary U (2^-62 integers)
+// qubits): the host multiplies them into one 16x16 unitary U (rounded once to
+// 2^-62 integers)
 // and the pass computes y = U x for every "row" x, the 16 amplitudes that
 // differ only in the window bits.
 //
