@@ -1191,8 +1191,8 @@ int fx_shape_launch(const FxShapeParams& P, cudaStream_t stream) {
   return check_cuda(cudaGetLastError());
 }
 
-// Double-double complex arithmetic for the pass unitary: products of the
-// gates' FP64 entries carried to ~106 bits with FMA-based error-free
+// Double-double complex arithmetic for the tables of the phase passes: products
+// of the gates' FP64 entries carried to ~106 bits with FMA-based error-free
 // transformations, the same on every host.
 struct Dd {
   double hi = 0.0, lo = 0.0;
@@ -1850,7 +1850,7 @@ void plan_tensor_block(const std::vector<HostOp>& ops, int n, const FxBlock& who
 // not touch them: the pass costs the same, and the sweep of its own goes
 // (n = 22: 36 us for a depolarizing channel, 23 for a dephasing one, beside
 // 30 for the pass).  Two layers with a channel per qubit, 11 qubits: 1065 ->
-// 665 us a call; 8 qubits, error against 80-bit
+// 710 us a call; 8 qubits, error against 80-bit
 // arithmetic 4.4e-16 -> 3.7e-16.  Never a pass of channels alone: it would
 // hold their rows to a shared exponent that no gate asks for, and gain little
 // (30 us against two sweeps).

@@ -1,7 +1,7 @@
 """The pass unitary of a window of many gates: outputs bit for bit those of the
 integer model whose U is the gates' exact product, rounded once to 2^-62.
 Gates with entries down to 2^-40, permutations, diagonals and signs among
-them; the host's product carries 2^-124."""
+them; the host's product carries 2^-91."""
 from fractions import Fraction
 
 import numpy as np
